@@ -2,6 +2,7 @@
 // FP64 direct sum (Traversal::direct, include/traversal.h:355-377).  Each
 // operator runs the same device kernel the solver uses, on a two- or few-cell
 // tree assembled from the caller's arrays.
+#include <algorithm>
 #include <cstring>
 #include <stdexcept>
 #include <string>
@@ -10,51 +11,115 @@
 #include "../../include/exafmm_b200.h"
 #include "fmm.h"
 #include "harmonics.cuh"
+#include "pair64.cuh"
 
 namespace exafmm_b200 {
 
 namespace {
 
-__global__ void k_direct(const double4 *tgt, long long nt, const double4 *src, long long ns, int prange,
-                         double cycle, double4 *trg) {
-  __shared__ double4 tile[256];
-  const long long i = blockIdx.x * (long long)blockDim.x + threadIdx.x;
-  double4 xi = make_double4(0, 0, 0, 0);
-  if (i < nt) xi = tgt[i];
-  double pot = 0, ax = 0, ay = 0, az = 0;
-  for (int ix = -prange; ix <= prange; ix++)
-    for (int iy = -prange; iy <= prange; iy++)
-      for (int iz = -prange; iz <= prange; iz++) {
-        const double sx = ix * cycle, sy = iy * cycle, sz = iz * cycle;
-        for (long long base = 0; base < ns; base += 256) {
-          __syncthreads();
-          if (base + threadIdx.x < ns) tile[threadIdx.x] = src[base + threadIdx.x];
-          __syncthreads();
-          const int cnt = (int)min((long long)256, ns - base);
-          for (int s = 0; s < cnt; s++) {
-            const double4 sj = tile[s];
-            const double dx = xi.x - sj.x - sx, dy = xi.y - sj.y - sy, dz = xi.z - sj.z - sz;
-            const double r2 = dx * dx + dy * dy + dz * dz;
-            if (r2 != 0.0) {
-              const double inv2 = 1.0 / r2;
-              const double qr = sj.w * sqrt(inv2);
-              const double s3 = inv2 * qr;
-              pot += qr;
-              ax += dx * s3;
-              ay += dy * s3;
-              az += dz * s3;
-            }
+// A block takes kDirThreads x TPL targets and a contiguous share of the source
+// tiles (kDirTile sources of one image each); with one share the sums are
+// added to the results, with more they are left in part[share][target] and
+// added in order by k_direct_add, so the result does not depend on timing.
+// Bound: the FP64 pipe, 18 operations a pair (pair64.cuh).  4,096 targets x
+// 1,000,003 sources kept 16 of the 148 SMs busy with one thread per target and
+// every source (160 ms).
+constexpr int kDirThreads = 128, kDirTile = 256;
+
+template <int TPL, bool IMAGES>
+__global__ void __launch_bounds__(kDirThreads)
+k_direct(const double4 *tgt, long long nt, const double4 *src, long long ns, int prange, double cycle, double4 *trg,
+         double4 *part) {
+  __shared__ double2 sxy[kDirTile], szq[kDirTile];
+  const long long t0 = (long long)blockIdx.x * (kDirThreads * TPL) + threadIdx.x;
+  double x[TPL], y[TPL], z[TPL], acc[TPL][4];
+#pragma unroll
+  for (int u = 0; u < TPL; u++) {
+    const long long i = t0 + (long long)u * kDirThreads;
+    const double4 v = i < nt ? tgt[i] : make_double4(0, 0, 0, 0);
+    x[u] = v.x;
+    y[u] = v.y;
+    z[u] = v.z;
+#pragma unroll
+    for (int k = 0; k < 4; k++) acc[u][k] = 0.0;
+  }
+  const long long per = (ns + kDirTile - 1) / kDirTile;  // tiles of one image
+  const int nb = 2 * prange + 1;
+  const long long tiles = per * nb * nb * nb;
+  const long long lo = tiles * blockIdx.y / gridDim.y, hi = tiles * (blockIdx.y + 1) / gridDim.y;
+  for (long long t = lo; t < hi; t++) {
+    const long long img = IMAGES ? t / per : 0, base = (IMAGES ? t - img * per : t) * kDirTile;
+    double sx = 0, sy = 0, sz = 0;
+    if (IMAGES) {
+      sx = (double)(img / (nb * nb) - prange) * cycle;
+      sy = (double)((img / nb) % nb - prange) * cycle;
+      sz = (double)(img % nb - prange) * cycle;
+    }
+    const int cnt = (int)min((long long)kDirTile, ns - base);
+    __syncthreads();
+    for (int k = threadIdx.x; k < kDirTile; k += kDirThreads) {  // past the end: far away, no charge
+      const double4 s = k < cnt ? src[base + k] : make_double4(1e18, 1e18, 1e18, 0.0);
+      sxy[k] = make_double2(s.x, s.y);
+      szq[k] = make_double2(s.z, s.w);
+    }
+    __syncthreads();
+    const int steps = (cnt + 1) / 2;
+    for (int s = 0; s < steps; s++) {
+      double dx[2 * TPL], dy[2 * TPL], dz[2 * TPL], q[2 * TPL];
+#pragma unroll
+      for (int h = 0; h < 2; h++) {
+        const double2 a = sxy[2 * s + h], b = szq[2 * s + h];
+#pragma unroll
+        for (int u = 0; u < TPL; u++) {
+          const int i = 2 * u + h;
+          dx[i] = x[u] - a.x;
+          dy[i] = y[u] - a.y;
+          dz[i] = z[u] - b.x;
+          q[i] = b.y;
+          if (IMAGES) {
+            dx[i] -= sx;
+            dy[i] -= sy;
+            dz[i] -= sz;
           }
         }
       }
-  if (i < nt) {
-    double4 r = trg[i];
-    r.x += pot;
-    r.y -= ax;
-    r.z -= ay;
-    r.w -= az;
-    trg[i] = r;
+      pairs64<2 * TPL, 2>(dx, dy, dz, q, acc);
+    }
   }
+#pragma unroll
+  for (int u = 0; u < TPL; u++) {
+    const long long i = t0 + (long long)u * kDirThreads;
+    if (i >= nt) continue;
+    if (part) {
+      part[(long long)blockIdx.y * nt + i] = make_double4(acc[u][0], acc[u][1], acc[u][2], acc[u][3]);
+    } else {
+      double4 r = trg[i];
+      r.x += acc[u][0];
+      r.y -= acc[u][1];
+      r.z -= acc[u][2];
+      r.w -= acc[u][3];
+      trg[i] = r;
+    }
+  }
+}
+
+__global__ void k_direct_add(const double4 *part, int shares, long long nt, double4 *trg) {
+  const long long i = blockIdx.x * (long long)blockDim.x + threadIdx.x;
+  if (i >= nt) return;
+  double4 r = make_double4(0, 0, 0, 0);
+  for (int s = 0; s < shares; s++) {
+    const double4 v = part[(long long)s * nt + i];
+    r.x += v.x;
+    r.y += v.y;
+    r.z += v.z;
+    r.w += v.w;
+  }
+  double4 o = trg[i];
+  o.x += r.x;
+  o.y -= r.y;
+  o.z -= r.z;
+  o.w -= r.w;
+  trg[i] = o;
 }
 
 // The MD wrappers' cutoff sum (wrappers/md_distributed.cxx:407-461): every
@@ -117,7 +182,7 @@ struct Mini {
     void *p = nullptr;
     EXA_CUDA(cudaMalloc(&p, (n ? n : 1) * sizeof(T)));
     bufs.push_back(p);
-    if (n) EXA_CUDA(cudaMemcpyAsync(p, h, n * sizeof(T), cudaMemcpyHostToDevice, st));
+    if (n && h) EXA_CUDA(cudaMemcpyAsync(p, h, n * sizeof(T), cudaMemcpyHostToDevice, st));
     return (T *)p;
   }
   template <typename T>
@@ -153,11 +218,33 @@ void check_P(int P) {
 
 }  // namespace
 
+// Shares of the source tiles: as many as bring the grid to two rounds of the
+// blocks the GPU holds (one share once the target blocks alone do), at least
+// two tiles each.  part_alloc(n) gives n double4 of scratch on st, where it is needed.
+template <typename Alloc>
 void direct_fp64(const double4 *tgt, long long nt, const double4 *src, long long ns, int prange, double cycle,
-                 double4 *trg, cudaStream_t st) {
-  if (nt == 0) return;
-  k_direct<<<(int)((nt + 255) / 256), 256, 0, st>>>(tgt, nt, src, ns, prange, cycle, trg);
-  EXA_CHECK_LAUNCH();
+                 double4 *trg, cudaStream_t st, Alloc &&part_alloc) {
+  auto launch = [&](auto kernel, int tpl) {
+    int per_sm = 1;
+    EXA_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kernel, kDirThreads, 0));
+    const long long nb = 2LL * prange + 1;
+    const long long tiles = (ns + kDirTile - 1) / kDirTile * nb * nb * nb;
+    const long long tb = (nt + kDirThreads * tpl - 1) / (kDirThreads * tpl);
+    long long shares = 2LL * kNumSMs * std::max(1, per_sm) / std::max(1LL, tb);
+    shares = std::max(1LL, std::min(std::min(shares, tiles / 2), 65535LL));
+    double4 *part = shares > 1 ? part_alloc(shares * nt) : nullptr;
+    kernel<<<dim3((unsigned)tb, (unsigned)shares), kDirThreads, 0, st>>>(tgt, nt, src, ns, prange, cycle, trg, part);
+    EXA_CHECK_LAUNCH();
+    if (part) {
+      k_direct_add<<<(unsigned)((nt + 127) / 128), 128, 0, st>>>(part, (int)shares, nt, trg);
+      EXA_CHECK_LAUNCH();
+    }
+  };
+  // two targets a thread halve the shared-memory reads; one where the targets
+  // would not fill half of the wider blocks
+  const bool two = nt > kDirThreads;
+  if (prange > 0) two ? launch(k_direct<2, true>, 2) : launch(k_direct<1, true>, 1);
+  else two ? launch(k_direct<2, false>, 2) : launch(k_direct<1, false>, 1);
 }
 
 }  // namespace exafmm_b200
@@ -182,7 +269,7 @@ int exafmm_direct(const double *targets, long long nt, const double *sources, lo
     const double4 *t = m.up((const double4 *)targets, nt);
     const double4 *s = m.up((const double4 *)sources, ns);
     double4 *r = m.up((const double4 *)trg, nt);
-    direct_fp64(t, nt, s, ns, prange, cycle, r, m.st);
+    direct_fp64(t, nt, s, ns, prange, cycle, r, m.st, [&](long long n) { return m.up((const double4 *)nullptr, n); });
     m.down((double4 *)trg, r, nt);
   });
 }
@@ -195,7 +282,7 @@ int exafmm_direct_range(const double *targets, long long nt, const double *sourc
     const double4 *t = m.up((const double4 *)targets, nt);
     const double4 *s = m.up((const double4 *)sources, ns);
     double4 *r = m.up((const double4 *)trg, nt);
-    direct_fp64(t, nt, s, ns, prange, cycle, r, m.st);
+    direct_fp64(t, nt, s, ns, prange, cycle, r, m.st, [&](long long n) { return m.up((const double4 *)nullptr, n); });
     m.down((double4 *)trg, r, nt);
   });
 }

@@ -1,0 +1,51 @@
+"""Pair kernels on the GPU against the oracle's direct sum: the direct sum at the
+edges of its target blocks and source tiles, and the P2P kernels at the edges of
+their lane groups, segments and divided leaves (a tree of one leaf is P2P alone)."""
+import numpy as np
+import pytest
+
+pytestmark = pytest.mark.gpu
+
+# FP64: sums of up to a few thousand terms of either sign, each within a few ulp
+TOL64 = 1e-13
+# mixed: FP32 products (2^-24, the reciprocal square root 2^-22) of two-float
+# separations, summed with compensation; 1e-6 is the form's stated precision
+TOL32 = 1e-6
+
+
+def _rel(a, b):
+    return float(np.linalg.norm(a - b) / np.linalg.norm(b))
+
+
+@pytest.mark.parametrize("nt,ns,images", [(1, 1, 0), (1, 257, 0), (128, 255, 0), (129, 256, 0), (300, 1031, 0),
+                                          (257, 513, 0), (5, 40, 1), (130, 65, 1)])
+def test_direct_block_and_tile_edges(ex, oracle, nt, ns, images):
+    rng = np.random.default_rng(nt * 1009 + ns)
+    t, s = rng.uniform(-1, 1, (nt, 4)), rng.uniform(-1, 1, (ns, 4))
+    s[0, :3] = t[0, :3] if ns > 1 else s[0, :3]  # one pair at distance zero
+    got = ex.direct(t, s, images=images, theta=0.4)
+    assert _rel(got, oracle.direct(t, s, images=images, theta=0.4)) < TOL64
+
+
+@pytest.mark.parametrize("mixed", [False, True])
+@pytest.mark.parametrize("n", [2, 7, 8, 9, 12, 13, 16, 17, 24, 25, 32, 33, 49, 64, 65, 70, 97, 130, 257, 1000])
+def test_one_leaf_is_the_direct_sum(ex, oracle, n, mixed):
+    x = np.random.default_rng(n).uniform(-1, 1, (n, 4))
+    if n > 8:
+        x[3, :3] = x[7, :3]  # coincident bodies: no contribution
+    with ex.Fmm(P=4, ncrit=1024, precision=ex.MIXED if mixed else ex.FP64) as f:
+        f.set_bodies(x)
+        f.solve()
+        got = f.results()
+        again = f.solve() or f.results()
+    ref = oracle.direct(x, x)
+    assert _rel(got[:, 0], ref[:, 0]) < (TOL32 if mixed else TOL64)
+    assert _rel(got[:, 1:], ref[:, 1:]) < (TOL32 if mixed else TOL64)
+    assert np.array_equal(got, again)  # divided leaves add in a fixed order
+
+
+@pytest.mark.parametrize("d", [1e-100, 1e-150, 1e-155])
+def test_tiny_distances_keep_their_weight(ex, d):
+    """The squared distance down to a subnormal number (1e-310, good to about 1e-14 of itself)."""
+    got = ex.direct(np.zeros((1, 4)), np.array([[d, 0.0, 0.0, 1.0], [0.0, 0.0, 0.0, 5.0]]))
+    assert abs(got[0, 0] * d - 1.0) < 1e-10
