@@ -31,9 +31,6 @@ static std::atomic<long long> g_launches{0};
 void note_launch() { g_launches.fetch_add(1, std::memory_order_relaxed); }
 long long launch_count() { return g_launches.load(std::memory_order_relaxed); }
 
-void direct_fp64(const double4 *tgt, long long nt, const double4 *src, long long ns, int prange, double cycle,
-                 double4 *trg, cudaStream_t st);
-
 namespace {
 
 // Phase events of the last solve: ev[0..7] bound bounds, tree, upward, lists,
@@ -101,7 +98,7 @@ struct Engine {
   M2LGemmBufs gemm;         // class-grouped tile M2L (mixed form)
   DBuf<double2> lat;        // periodic lattice: supercell multipoles and warp partials
   DBuf<double> dip;         // dipole reduction scratch and result
-  P2PWork p2pw;               // work counters and order of the mixed P2P kernels
+  P2PWork p2pw;               // work queue of the P2P kernels
   DBuf<double4> trg, out;
   Timing tm;
   bool tree_ok = false, up_ok = false, lists_ok = false;
@@ -395,7 +392,7 @@ struct Engine {
       rel_bodies32(a, jsrc->C.tree.xyzq_tree.p, ns, x32j.p);
       p2p_mixed(C, a, x32.p, false, p2pw, x32j.p);
     } else {
-      p2p_fp64(a);
+      p2p_fp64(C, a, false, p2pw);
     }
   }
 
@@ -464,7 +461,7 @@ struct Engine {
         rel_bodies32(a, x32.p);
         p2p_mixed(C, a, x32.p, C.prm.images > 0, p2pw);
       } else {
-        p2p_fp64(a);
+        p2p_fp64(C, a, C.prm.images > 0, p2pw);
       }
     } else {
       EXA_CUDA(cudaEventRecord(tm.ev[4], C.stream));

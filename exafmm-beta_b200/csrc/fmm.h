@@ -43,6 +43,10 @@ void m2m_fp64(const FmmArgs &a, int level, long long nodes_at_level);
 void m2l_fp64(const FmmArgs &a, int skip_min_level = -1, int skip_max_dl = 0);
 void l2l_fp64(const FmmArgs &a, int level, long long nodes_at_level);
 void l2p_fp64(const FmmArgs &a);
+struct P2PWork;
+// FP64 P2P (p2p64.cu); periodic: the lists hold image pairs.
+void p2p_fp64(Context &C, const FmmArgs &a, bool periodic, P2PWork &w);
+// The same without a work queue: one operator call on a few cells.
 void p2p_fp64(const FmmArgs &a);
 
 // Mixed form: FP32 M2L for targets at level >= kMixedMinLevel and source/target
@@ -107,31 +111,18 @@ void dipole_correction_fp64(const double4 *xt, double4 *trg, long long n, double
                             double nbodies, cudaStream_t st);
 
 // Mixed-precision P2P (p2p32.cu): bodies as two-float pairs relative to the
-// root center; periodic selects the form that tests every pair for r = 0.
+// root center; periodic: the lists hold image pairs.
 void rel_bodies32(const FmmArgs &a, float4 *x32);
 // The same for other bodies (a separate source tree's) about the root center of a.
 void rel_bodies32(const FmmArgs &a, const double4 *xt, long long n, float4 *x32);
-// Scratch of the mixed P2P: the persistent kernels' work counters and their
-// work order (target leaves by kind, longest first).
+// Work queue of the P2P kernels (p2p_work.cuh).
 struct P2PWork {
-  DBuf<unsigned long long> next;   // [2] work counters
-  DBuf<unsigned> key, key_alt;     // order keys
-  DBuf<int> order, order_alt;      // cells in work order
-  DBuf<int> count;                 // [3] leaves of each kind: two targets per lane, three, no P2P list
-  // The three-target kind runs on a stream of its own, forked from and joined
-  // back to the solve's stream, so its blocks take the SMs that the
-  // two-target kind's last leaves leave idle (made on first use).
-  cudaStream_t side = nullptr;
-  cudaEvent_t fork = nullptr, join = nullptr;
-  P2PWork() = default;
-  P2PWork(const P2PWork &) = delete;
-  P2PWork &operator=(const P2PWork &) = delete;
-  ~P2PWork() {
-    if (side) cudaStreamSynchronize(side);
-    if (fork) cudaEventDestroy(fork);
-    if (join) cudaEventDestroy(join);
-    if (side) cudaStreamDestroy(side);
-  }
+  DBuf<int4> items;           // items of the cost classes
+  DBuf<int4> leaf;            // per leaf: sources of a segment, items, segments, targets per lane
+  DBuf<int> nsrc;             // per leaf: sources
+  DBuf<int> count;            // items of each class
+  DBuf<double4> scratch;      // segment sums of divided leaves
+  DBuf<unsigned char> zero;   // total cost, work counter and per-leaf progress, cleared together
 };
 // x32j (null: x32) holds the source bodies, whose cells are a.src_cell_b when set.
 void p2p_mixed(Context &C, const FmmArgs &a, const float4 *x32, bool periodic, P2PWork &w,

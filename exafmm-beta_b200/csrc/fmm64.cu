@@ -1,4 +1,4 @@
-// FP64 expansion operators: P2M, M2M, M2L, L2L, L2P, P2P (kernels/laplace.h:150-388),
+// FP64 expansion operators: P2M, M2M, M2L, L2L, L2P (kernels/laplace.h:237-388),
 // one warp per cell, in the conventions of harmonics.cuh.
 #include <algorithm>
 
@@ -427,81 +427,6 @@ __global__ void k_l2p(DevTables t, const int4 *cell_b, const double4 *cell_x, co
   }
 }
 
-// ---------------------------------------------------------------- P2P
-// pot += q/r, grad += q (x_j - x_i)/r^3 with r = 0 pairs skipped (laplace.h:150-235).
-template <int TPL>
-__global__ void k_p2p(const int *off, const int *src, long long ncells, const int4 *cell_b, const double4 *xt,
-                      const int4 *cell_bj, const double4 *xtj, double4 *trg, double cycle) {
-  __shared__ double4 sbuf[kWarpsPerBlock][32];
-  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-  for (long long c = (long long)blockIdx.x * kWarpsPerBlock + warp; c < ncells; c += (long long)gridDim.x * kWarpsPerBlock) {
-    const int b = off[c], e = off[c + 1];
-    if (b == e) continue;
-    const int4 ci = cell_b[c];
-    for (int tb = 0; tb < ci.y; tb += 32 * TPL) {
-      double xi[TPL], yi[TPL], zi[TPL], pot[TPL], ax[TPL], ay[TPL], az[TPL];
-#pragma unroll
-      for (int u = 0; u < TPL; u++) {
-        const int i = tb + lane + 32 * u;
-        double4 v = make_double4(0, 0, 0, 0);
-        if (i < ci.y) v = xt[ci.x + i];
-        xi[u] = v.x;
-        yi[u] = v.y;
-        zi[u] = v.z;
-        pot[u] = ax[u] = ay[u] = az[u] = 0.0;
-      }
-      for (int q = b; q < e; q++) {
-        const int packed = src[q];
-        const int cj = packed & 0x3ffffff, img = packed >> 26;
-        double sx, sy, sz;
-        image_shift(img, cycle, sx, sy, sz);
-        const int4 cjb = cell_bj[cj];
-        for (int sb = 0; sb < cjb.y; sb += 32) {
-          const int ns = min(32, cjb.y - sb);
-          if (lane < ns) {
-            double4 s = xtj[cjb.x + sb + lane];
-            s.x += sx;
-            s.y += sy;
-            s.z += sz;
-            sbuf[warp][lane] = s;
-          }
-          __syncwarp();
-          for (int s = 0; s < ns; s++) {
-            const double4 sj = sbuf[warp][s];
-#pragma unroll
-            for (int u = 0; u < TPL; u++) {
-              const double dx = xi[u] - sj.x, dy = yi[u] - sj.y, dz = zi[u] - sj.z;
-              const double r2 = dx * dx + dy * dy + dz * dz;
-              if (r2 != 0.0) {
-                const double inv = rsqrt(r2);
-                const double qr = sj.w * inv;
-                const double qr3 = qr * inv * inv;
-                pot[u] += qr;
-                ax[u] = fma(dx, qr3, ax[u]);
-                ay[u] = fma(dy, qr3, ay[u]);
-                az[u] = fma(dz, qr3, az[u]);
-              }
-            }
-          }
-          __syncwarp();
-        }
-      }
-#pragma unroll
-      for (int u = 0; u < TPL; u++) {
-        const int i = tb + lane + 32 * u;
-        if (i < ci.y) {
-          double4 r = trg[ci.x + i];
-          r.x += pot[u];
-          r.y -= ax[u];
-          r.z -= ay[u];
-          r.w -= az[u];
-          trg[ci.x + i] = r;
-        }
-      }
-    }
-  }
-}
-
 // ---------------------------------------------------------------- periodic lattice
 // Traversal::traversePeriodic (traversal.h:233-287).  The root multipole is
 // replicated over a supercell of nb^3 copies (nb = 2 prange + 1).  Each lattice
@@ -750,22 +675,6 @@ void l2p_fp64(const FmmArgs &a) {
   set_smem(k_l2p, smem);
   k_l2p<<<blocks_for(a.ncells), 32 * kWarpsPerBlock, smem, a.stream>>>(t, a.cell_b, a.cell_x, a.xt, a.L64,
                                                                        a.trg64, a.ncells);
-  EXA_CHECK_LAUNCH();
-}
-
-void p2p_fp64(const FmmArgs &a) {
-  const int tpl = (a.ncrit + 31) / 32;
-  const int4 *bj = a.src_cell_b ? a.src_cell_b : a.cell_b;
-  const double4 *xj = a.src_xt ? a.src_xt : a.xt;
-  if (tpl <= 1)
-    k_p2p<1><<<blocks_for(a.ncells), 32 * kWarpsPerBlock, 0, a.stream>>>(a.p2p_off, a.p2p_src, a.ncells, a.cell_b,
-                                                                          a.xt, bj, xj, a.trg64, a.cycle);
-  else if (tpl <= 2)
-    k_p2p<2><<<blocks_for(a.ncells), 32 * kWarpsPerBlock, 0, a.stream>>>(a.p2p_off, a.p2p_src, a.ncells, a.cell_b,
-                                                                          a.xt, bj, xj, a.trg64, a.cycle);
-  else
-    k_p2p<4><<<blocks_for(a.ncells), 32 * kWarpsPerBlock, 0, a.stream>>>(a.p2p_off, a.p2p_src, a.ncells, a.cell_b,
-                                                                          a.xt, bj, xj, a.trg64, a.cycle);
   EXA_CHECK_LAUNCH();
 }
 

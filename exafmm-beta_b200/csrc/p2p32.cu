@@ -31,10 +31,7 @@
 // bounds this kernel.  The rsqrt flushes subnormal inputs, so a pair closer
 // than about 1e-19 (an r^2 below the FP32 normal range) also contributes
 // nothing; such inputs need the FP64 plain method.
-#include <algorithm>
-#include <stdexcept>
-
-#include "fmm.h"
+#include "p2p_work.cuh"
 
 namespace exafmm_b200 {
 namespace {
@@ -219,49 +216,22 @@ __device__ __forceinline__ void pair_step(const Stage &sm, int p, const Targets<
   }
 }
 
-// Streams the bodies of the P2P list entries [qb, qe) through the warp and
-// accumulates their action on the lane's targets into `acc`.
-template <int S, int TPL, bool PERIODIC>
-__device__ __forceinline__ void p2p_stream(Stage &sm, const int *src, const int4 *cell_b, const float4 *x32,
-                                           double cycle, int qb, int qe, const Targets<TPL> &T, Sums<TPL> &acc) {
-  constexpr int G = 32 / S, CH = 32 * G;
-  const int lane = threadIdx.x & 31, g = lane / S;
-  int q = qb, o = 0, qw = qb - 64;
-  int w_start = 0, w_size = 0, w_img = 13;
+// Streams the segment's bodies through the warp and accumulates their action
+// on the lane's targets into `acc`.  One body of code for every group width: with
+// one per width (S a template parameter) the warps of an SM, each at its own
+// width, missed the instruction cache (4M-body P2P 28.3 against 20.3 ms).
+template <int TPL, bool PERIODIC>
+__device__ __forceinline__ void p2p_stream(int lS, Stage &sm, P2PState &st, const int *src,
+                                           const int4 *cell_b, const float4 *x32, double cycle, const Targets<TPL> &T,
+                                           Sums<TPL> &acc) {
+  const int lane = threadIdx.x & 31, G = 32 >> lS;
   for (;;) {
-    // ---- fill one chunk (warp-uniform walk over the segments) ----
-    int filled = 0;
-    while (filled < CH && q < qe) {
-      if (q - qw >= 32) {  // next window of 32 segment descriptors, one per lane
-        qw = q;
-        const int qq = qw + lane;
-        w_start = 0;
-        w_size = 0;
-        w_img = 13;
-        if (qq < qe) {
-          const int packed = src[qq];
-          const int4 cb = cell_b[packed & 0x3ffffff];
-          w_start = cb.x;
-          w_size = cb.y;
-          w_img = packed >> 26;
-        }
-      }
-      const int l = q - qw;
-      const int start = __shfl_sync(kFull, w_start, l);
-      const int size = __shfl_sync(kFull, w_size, l);
-      const int img = PERIODIC ? __shfl_sync(kFull, w_img, l) : 13;
-      const int m = min(CH - filled, size - o);
-      for (int k = lane; k < m; k += 32) stage_body<PERIODIC>(sm, filled + k, x32, (long long)start + o + k, img, cycle);
-      filled += m;
-      o += m;
-      if (o == size) {
-        q++;
-        o = 0;
-      }
-    }
+    const int filled = p2p_fill(st, 32 * G, src, cell_b, [&](int k, long long body, int img) {
+      stage_body<PERIODIC>(sm, k, x32, body, img, cycle);
+    });
     if (filled == 0) break;
-    const int steps = (filled + 2 * G - 1) / (2 * G);  // pair steps per group
-    const int padded = 2 * G * (steps + (steps & 1));   // even step count for the unrolled loop
+    const int steps = (filled + 2 * G - 1) >> (6 - lS);  // pair steps per group
+    const int padded = 2 * G * (steps + (steps & 1));    // even step count for the unrolled loop
     for (int k = filled + lane; k < padded; k += 32) stage_dummy(sm, k);
     __syncwarp();
 
@@ -269,6 +239,7 @@ __device__ __forceinline__ void p2p_stream(Stage &sm, const int *src, const int4
     f2p pp[TPL], px[TPL], py[TPL], pz[TPL];
 #pragma unroll
     for (int u = 0; u < TPL; u++) pp[u] = px[u] = py[u] = pz[u] = 0ull;
+    const int g = lane >> lS;
     for (int s = 0; s < steps; s += 2) {
       pair_step(sm, g + G * s, T, pp, px, py, pz);
       pair_step(sm, g + G * (s + 1), T, pp, px, py, pz);
@@ -285,149 +256,91 @@ __device__ __forceinline__ void p2p_stream(Stage &sm, const int *src, const int4
   }
 }
 
-// One pass over the leaf's source stream for its targets [tb, tb + S * TPL).
-template <int S, int TPL, bool PERIODIC>
-__device__ __forceinline__ void p2p_pass(Stage &sm, int4 cb, int tb, int b, int e, const int *src,
+// One pass over the item's segments for the leaf's targets from st.tb on.
+template <int TPL, bool PERIODIC>
+__device__ __forceinline__ void p2p_pass(int lS, Stage &sm, P2PState &st, const P2PItems &w, const int *src,
                                          const int4 *cell_bj, const float4 *x32, const float4 *x32j, double4 *trg,
                                          double cycle) {
-  const int lane = threadIdx.x & 31, g = lane / S, j = lane % S;
-  {
-    Targets<TPL> T;
+  const int lane = threadIdx.x & 31;
+  Targets<TPL> T;
 #pragma unroll
-    for (int u = 0; u < TPL; u++) {
-      const int i = tb + j + S * u;
-      float4 h = make_float4(0.f, 0.f, 0.f, 0.f), l = h;
-      if (i < cb.y) {
-        h = x32[2 * ((long long)cb.x + i)];
-        l = x32[2 * ((long long)cb.x + i) + 1];
-      }
-      T.t[u][0] = pk2(h.x, h.x);
-      T.t[u][1] = pk2(h.y, h.y);
-      T.t[u][2] = pk2(h.z, h.z);
-      T.t[u][3] = pk2(l.x, l.x);
-      T.t[u][4] = pk2(l.y, l.y);
-      T.t[u][5] = pk2(l.z, l.z);
+  for (int u = 0; u < TPL; u++) {
+    const int i = st.tb + (lane & ((1 << lS) - 1)) + (u << lS);
+    float4 h = make_float4(0.f, 0.f, 0.f, 0.f), l = h;
+    if (i < st.cb.y) {
+      h = x32[2 * ((long long)st.cb.x + i)];
+      l = x32[2 * ((long long)st.cb.x + i) + 1];
     }
+    T.t[u][0] = pk2(h.x, h.x);
+    T.t[u][1] = pk2(h.y, h.y);
+    T.t[u][2] = pk2(h.z, h.z);
+    T.t[u][3] = pk2(l.x, l.x);
+    T.t[u][4] = pk2(l.y, l.y);
+    T.t[u][5] = pk2(l.z, l.z);
+  }
+  p2p_seek(st, st.item.y, src, cell_bj);
+  if (lane == 0) st.at = st.item.y;
+  __syncwarp();
+  while (st.at < st.item.z) {
+    if (lane == 0) st.pos.w = min(st.seg, st.item.z - st.at);
+    __syncwarp();
     Sums<TPL> acc;
-    p2p_stream<S, TPL, PERIODIC>(sm, src, cell_bj, x32j, cycle, b, e, T, acc);
+    p2p_stream<TPL, PERIODIC>(lS, sm, st, src, cell_bj, x32j, cycle, T, acc);
     // combine the groups (lanes j, j + S, j + 2S, ... hold the same targets) in FP64
 #pragma unroll
     for (int u = 0; u < TPL; u++) {
       double v[4];
 #pragma unroll
       for (int k = 0; k < 4; k++) v[k] = (double)acc.k[u][k].s - (double)acc.k[u][k].c;
-#pragma unroll
-      for (int off = S; off < 32; off <<= 1)
+#pragma unroll 1
+      for (int off = 1 << lS; off < 32; off <<= 1)
 #pragma unroll
         for (int k = 0; k < 4; k++) v[k] += __shfl_xor_sync(kFull, v[k], off);
-      const int i = tb + j + S * u;
-      if (g == 0 && i < cb.y) {
-        double4 r = trg[cb.x + i];
-        r.x += v[0];
-        r.y -= v[1];
-        r.z -= v[2];
-        r.w -= v[3];
-        trg[cb.x + i] = r;
-      }
+      if (lane < (1 << lS)) p2p_store(w, st, lane + (u << lS), v, trg);
     }
+    __syncwarp();
+    if (lane == 0) st.at += st.seg;
+    __syncwarp();
   }
 }
 
 // Target slots of a leaf: passes of S lanes x TPL targets per lane, each pass
 // taking the narrowest group that holds the targets still left (S = 32 while
-// more than 16 TPL remain).  A 70-body leaf at two per lane: 64 + 8 slots in
-// two passes, rather than 96 at three per lane or 128 in two full passes.
-// Every pass streams the leaf's sources again, which costs about as much as
-// a few more target slots, so a leaf takes three targets per lane when that
-// costs fewer slots plus passes.  The two kinds run as separate kernels, so
-// the three-target code's registers do not lower the occupancy of the
-// two-target one.
-__host__ __device__ __forceinline__ int pass_lanes(int left, int tpl) {
-  return left <= 4 * tpl ? 4 : left <= 8 * tpl ? 8 : left <= 16 * tpl ? 16 : 32;
-}
-constexpr int kPassCharge = 4;  // target slots one more stream of the sources costs
-__host__ __device__ __forceinline__ int pass_cost(int n, int tpl) {
-  int cost = 0;
-  for (int tb = 0; tb < n;) {
-    const int w = pass_lanes(n - tb, tpl) * tpl;
-    cost += w + kPassCharge;
-    tb += w;
-  }
-  return cost;
-}
-__device__ __forceinline__ bool three_per_lane(int n) { return pass_cost(n, 3) < pass_cost(n, 2); }
-
-// Work order: each cell's kind (0: a leaf of two targets per lane, 1: three,
-// 2: no P2P list; tpl 2 or 3 gives every leaf that kind, tpl 0 chooses by the
-// leaf's size) above its cost (its bodies times the bodies of its list,
-// capped), reversed so that an ascending sort puts the costliest leaf of
-// each kind first.  count[kind] receives the cells of each kind.
-constexpr int kCostBits = 22;
-constexpr unsigned kCostMax = (1u << kCostBits) - 1;
-
-__global__ void k_p2p_keys(const int *off, const int *src, long long ncells, const int4 *cell_b,
-                           const int4 *cell_bj, int tpl, unsigned *key, int *val, int *count) {
-  for (long long c = blockIdx.x * (long long)blockDim.x + threadIdx.x; c < ncells;
-       c += (long long)gridDim.x * blockDim.x) {
-    const int b = off[c], e = off[c + 1];
-    unsigned kind = 2, cost = 0;
-    if (b < e) {
-      const int nb = cell_b[c].y;
-      unsigned long long s = 0;
-      for (int q = b; q < e; q++) s += (unsigned)cell_bj[src[q] & 0x3ffffff].y;
-      kind = (tpl == 0 ? three_per_lane(nb) : tpl == 3) ? 1u : 0u;
-      cost = (unsigned)min((unsigned long long)kCostMax, s * (unsigned long long)nb);
-    }
-    key[c] = (kind << kCostBits) | (kCostMax - cost);
-    val[c] = (int)c;
-    atomicAdd(&count[kind], 1);
-  }
-}
-
+// more than 16 TPL remain; pass_log_lanes).  A 70-body leaf at two per lane: 64 + 8
+// slots in two passes, rather than 96 at three per lane or 128 in two full
+// passes.  Every pass streams the leaf's sources again, which costs about as
+// much as kPassCharge more target slots, so a leaf takes three targets per
+// lane when that costs fewer slots plus passes (targets_per_lane).
+//
 // Persistent one-warp blocks, as many as fit on the GPU; each takes the next
-// target leaf of its kind from a counter, in the work order above (longest
-// first), until none is left, so leaves of very different cost balance out
-// and the warps finish together.  A leaf's result does not depend on when or
-// by which warp it is evaluated.
-// Resident warps per SM: the register budgets (96 and 126 registers, no
-// spills) at which the two kinds measured fastest on a 512-system batch at
-// P = 10 (P2P 55.3 -> 54.5 ms against 16 and 12 warps; the same on one 4M
-// solve).
-constexpr int kWarps2 = 20, kWarps3 = 16;
+// item from the queue (p2p_work.cuh) until none is left.  A leaf's result does
+// not depend on when or by which warps it is evaluated.  One kernel for leaves
+// of two and of three targets per lane: as two kernels (20 and 16 warps per
+// SM), the second one's blocks could only start when the first one's ended, and
+// each had a tail of its own.
+constexpr int kWarps32 = 16;       // resident warps per SM
+constexpr int kSegCost32 = 16384;  // slots x sources of a stream's smallest segment
 
-template <bool PERIODIC, int TPL>
-__global__ void __launch_bounds__(32, TPL == 2 ? kWarps2 : kWarps3)
-k_p2p32(const int *off, const int *src, const int *order, const int *count, const int4 *cell_b,
-        const int4 *cell_bj, const float4 *x32, const float4 *x32j, double4 *trg, double cycle,
-        unsigned long long *next) {
+template <bool PERIODIC>
+__global__ void __launch_bounds__(32, kWarps32)
+k_p2p32(P2PItems w, const int *off, const int *src, const int4 *cell_b, const int4 *cell_bj, const float4 *x32,
+        const float4 *x32j, double4 *trg, double cycle) {
   __shared__ Stage sm;
-  const long long items = count[TPL == 2 ? 0 : 1];
-  const int *mine = order + (TPL == 2 ? 0 : count[0]);
-  for (;;) {
-    unsigned long long k = 0;
-    if (threadIdx.x == 0) k = atomicAdd(next, 1ull);
-    k = __shfl_sync(kFull, k, 0);
-    if ((long long)k >= items) return;
-    const int c = mine[k];
-    const int b = off[c], e = off[c + 1];
-    const int4 cb = cell_b[c];
-    for (int tb = 0; tb < cb.y;) {
-      const int left = cb.y - tb;
-      if (left <= 4 * TPL) {
-        p2p_pass<4, TPL, PERIODIC>(sm, cb, tb, b, e, src, cell_bj, x32, x32j, trg, cycle);
-        tb += 4 * TPL;
-      } else if (left <= 8 * TPL) {
-        p2p_pass<8, TPL, PERIODIC>(sm, cb, tb, b, e, src, cell_bj, x32, x32j, trg, cycle);
-        tb += 8 * TPL;
-      } else if (left <= 16 * TPL) {
-        p2p_pass<16, TPL, PERIODIC>(sm, cb, tb, b, e, src, cell_bj, x32, x32j, trg, cycle);
-        tb += 16 * TPL;
-      } else {
-        p2p_pass<32, TPL, PERIODIC>(sm, cb, tb, b, e, src, cell_bj, x32, x32j, trg, cycle);
-        tb += 32 * TPL;
-      }
-      __syncwarp();  // the stage buffer is free before the next pass's first fill
-    }
+  __shared__ P2PState state;
+  P2PState &st = state;
+  int4 item;
+  while (p2p_next(w, item)) {
+    const int4 lf = w.leaf[item.x];
+    p2p_begin(st, item, lf.x, lf.w, off, cell_b);
+    if (lf.w == 2)
+      p2p_passes(st, 2, [&](int lS) {
+        p2p_pass<2, PERIODIC>(lS, sm, st, w, src, cell_bj, x32, x32j, trg, cycle);
+      });
+    else
+      p2p_passes(st, 3, [&](int lS) {
+        p2p_pass<3, PERIODIC>(lS, sm, st, w, src, cell_bj, x32, x32j, trg, cycle);
+      });
+    if (st.item.w >= 0) p2p_finish(w, st, trg);
   }
 }
 
@@ -450,50 +363,14 @@ void p2p_mixed(Context &C, const FmmArgs &a, const float4 *x32, bool periodic, P
   const long long nc = a.ncells;
   if (nc <= 0) return;
   cudaStream_t st = a.stream;
-  w.next.ensure(2);
-  w.count.ensure(3);
-  w.key.ensure(nc);
-  w.key_alt.ensure(nc);
-  w.order.ensure(nc);
-  w.order_alt.ensure(nc);
-  EXA_CUDA(cudaMemsetAsync(w.next.p, 0, 2 * sizeof(unsigned long long), st));
-  EXA_CUDA(cudaMemsetAsync(w.count.p, 0, 3 * sizeof(int), st));
-  const int kg = (int)std::max<long long>(1, std::min<long long>((long long)kNumSMs * 8, (nc + 255) / 256));
-  k_p2p_keys<<<kg, 256, 0, st>>>(a.p2p_off, a.p2p_src, nc, a.cell_b, cell_bj, C.prm.p2p_tpl, w.key.p, w.order.p,
-                                 w.count.p);
-  EXA_CHECK_LAUNCH();
-  const bool alt = radix_sort_u32(w.key.p, w.order.p, w.key_alt.p, w.order_alt.p, nc, 0, kCostBits + 2, C.sort,
-                                  C.err.p, st);
-  const int *order = alt ? w.order_alt.p : w.order.p;
-  const unsigned g2 = (unsigned)std::min<long long>(nc, (long long)kNumSMs * kWarps2);
-  const unsigned g3 = (unsigned)std::min<long long>(nc, (long long)kNumSMs * kWarps3);
-  if (!w.side) {
-    int dev = 0;
-    EXA_CUDA(cudaGetDevice(&dev));
-    EXA_CUDA(cudaStreamCreateWithFlags(&w.side, cudaStreamNonBlocking));
-    EXA_CUDA(cudaEventCreateWithFlags(&w.fork, cudaEventDisableTiming));
-    EXA_CUDA(cudaEventCreateWithFlags(&w.join, cudaEventDisableTiming));
-  }
-  // the two kinds write disjoint target leaves; the side stream starts after
-  // the work order is sorted and the solve's stream waits for it at the end
-  EXA_CUDA(cudaEventRecord(w.fork, st));
-  EXA_CUDA(cudaStreamWaitEvent(w.side, w.fork, 0));
-  if (periodic) {
-    k_p2p32<true, 2><<<g2, 32, 0, st>>>(a.p2p_off, a.p2p_src, order, w.count.p, a.cell_b, cell_bj, x32, x32j,
-                                        a.trg64, a.cycle, w.next.p);
+  const P2PItems q = p2p_plan(C, a, w, C.prm.p2p_tpl, kNumSMs * kWarps32, kSegCost32);
+  const unsigned grid = (unsigned)std::min<long long>(q.cap, (long long)kNumSMs * kWarps32);
+  auto launch = [&](auto kernel) {
+    kernel<<<grid, 32, 0, st>>>(q, a.p2p_off, a.p2p_src, a.cell_b, cell_bj, x32, x32j, a.trg64, a.cycle);
     EXA_CHECK_LAUNCH();
-    k_p2p32<true, 3><<<g3, 32, 0, w.side>>>(a.p2p_off, a.p2p_src, order, w.count.p, a.cell_b, cell_bj, x32, x32j,
-                                            a.trg64, a.cycle, w.next.p + 1);
-  } else {
-    k_p2p32<false, 2><<<g2, 32, 0, st>>>(a.p2p_off, a.p2p_src, order, w.count.p, a.cell_b, cell_bj, x32, x32j,
-                                         a.trg64, a.cycle, w.next.p);
-    EXA_CHECK_LAUNCH();
-    k_p2p32<false, 3><<<g3, 32, 0, w.side>>>(a.p2p_off, a.p2p_src, order, w.count.p, a.cell_b, cell_bj, x32, x32j,
-                                             a.trg64, a.cycle, w.next.p + 1);
-  }
-  EXA_CHECK_LAUNCH();
-  EXA_CUDA(cudaEventRecord(w.join, w.side));
-  EXA_CUDA(cudaStreamWaitEvent(st, w.join, 0));
+  };
+  if (periodic) launch(k_p2p32<true>);
+  else launch(k_p2p32<false>);
 }
 
 }  // namespace exafmm_b200
