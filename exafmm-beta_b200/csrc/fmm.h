@@ -88,9 +88,11 @@ struct M2LGemmBufs {
   DBuf<int> pval, pval_alt;           // their list positions
   DBuf<int> cstart, cbase;            // class ranges, chunk offsets per class
   DBuf<float> Y;                      // per list entry: the pair's contribution (real dofs)
+  DBuf<double> K64, Ms64r, Y64;       // the FP64 products' operators, multipoles and contributions
   DBuf<int> cnt;
   DBuf<int> left_cnt, left_off, left_src;
   DBuf<int> comp_cnt, comp_off, comp_src;  // pairs outside the mixed policy (FP64), per target
+  bool fp64 = false;          // FP64 products (plain method), every pair
   bool force = false;         // use the class products whatever the size (parity tests)
   bool tensor_cores = true;   // tcgen05 bf16x3 products, else FP32 on the CUDA cores
   bool tma = true;            // P = 8 on the tensor cores: source pieces gathered by TMA

@@ -38,6 +38,9 @@
 // tcgen05.mma into an FP32 accumulator in tensor memory: the terms left out
 // weigh about 2^-24, FP32 rounding.  The CUDA-core one (k_m2l_class_gemm) is a
 // plain FP32 product.
+//
+// The plain method takes the same route in FP64 (k_m2l_class_gemm64): every
+// pair, operators, multipoles, products and contributions in FP64.
 #include <cuda.h>
 #include <cuda_bf16.h>
 
@@ -128,7 +131,7 @@ __device__ __forceinline__ unsigned long long class_key_image(int lt, int dl, in
 // 1. Per pair of the target-grouped list: its class's hash slot, or -1.
 __global__ void k_pair_class(const int *off, const int *src, long long ncells, const double4 *cell_x,
                              const int2 *cell_pl, int min_level, int max_dl, unsigned long long *hk,
-                             long long hmask, int *pair_slot) {
+                             long long hmask, int *pair_slot, const int *sys_cell, int nsys, long long min_pairs) {
   const int lane = threadIdx.x & 31;
   const long long warps = (long long)gridDim.x * (blockDim.x >> 5);
   for (long long c = (long long)blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5); c < ncells; c += warps) {
@@ -136,13 +139,24 @@ __global__ void k_pair_class(const int *off, const int *src, long long ncells, c
     if (b == e) continue;
     const double4 Xt = cell_x[c];
     const int lt = cell_pl[c].y;
+    // a forest's system takes part by its own pair count, as its solo solve does
+    bool part = true;
+    if (sys_cell) {
+      int lo = 0, hi = nsys - 1;  // last s with sys_cell[s] <= c
+      while (lo < hi) {
+        const int mid = (lo + hi + 1) >> 1;
+        if (sys_cell[mid] <= c) lo = mid;
+        else hi = mid - 1;
+      }
+      part = off[sys_cell[lo + 1]] - off[sys_cell[lo]] >= min_pairs;
+    }
     for (int q = b + lane; q < e; q += 32) {
       const int packed = src[q];
       const int cj = packed & 0x3ffffff, img = packed >> 26;
       const int ls = cell_pl[cj].y;
       const int dl = ls - lt;
       int slot = -1;
-      if (lt >= min_level && lt < 32 && dl <= max_dl && dl >= -max_dl) {
+      if (part && lt >= min_level && lt < 32 && dl <= max_dl && dl >= -max_dl) {
         const double4 Xs = cell_x[cj];
         const double rmin = fmin(Xt.w, Xs.w);
         const double fx = rint((Xt.x - Xs.x) / rmin), fy = rint((Xt.y - Xs.y) / rmin), fz = rint((Xt.z - Xs.z) / rmin);
@@ -197,12 +211,12 @@ __global__ void k_class_ids(const int *cs_sorted, int ncls, int *hid) {
 // image (TMA).  NDP and the layout are template parameters so that mapping an
 // entry's position to its (output, input) pair is shifts and constant
 // divisions, not runtime divisions (the build was bound by integer work).
-enum KLayout : int { kKFp32 = 0, kKCore = 1, kKSwizzled = 2 };
+enum KLayout : int { kKFp32 = 0, kKCore = 1, kKSwizzled = 2, kKFp64 = 3 };
 
 template <int NDP, int LAYOUT>
 __global__ void __launch_bounds__(256)
-k_build_K(DevTables t, const unsigned long long *ck, int P, float *Kt, unsigned short *Kb, const double4 *cell_x,
-          double cycle) {
+k_build_K(DevTables t, const unsigned long long *ck, int P, float *Kt, unsigned short *Kb, double *Kd,
+          const double4 *cell_x, double cycle) {
   extern __shared__ double2 S[];  // S'_p^q, q >= 0, at d / R_t
   constexpr int KB = (NDP + 63) / 64;  // 128-byte K-blocks of the swizzled image
   constexpr int IMG = LAYOUT == kKSwizzled ? KB * NDP * 64 : NDP * NDP;
@@ -278,7 +292,9 @@ k_build_K(DevTables t, const unsigned long long *ck, int P, float *Kt, unsigned 
       }
       val = fn * (rp == 0 ? sr : si);
     }
-    if constexpr (LAYOUT == kKFp32) {
+    if constexpr (LAYOUT == kKFp64) {
+      Kd[(long long)blockIdx.x * NDP * NDP + c * NDP + r] = val;
+    } else if constexpr (LAYOUT == kKFp32) {
       Kt[(long long)blockIdx.x * NDP * NDP + c * NDP + r] = (float)val;
     } else {
       unsigned short h[3];
@@ -293,7 +309,7 @@ k_build_K(DevTables t, const unsigned long long *ck, int P, float *Kt, unsigned 
 // Scaled multipoles over real degrees of freedom, padded to NDP: FP32 rows
 // (Msr[cell][dof]), or three bf16 pieces per cell (Msb[cell][piece][dof]).
 __global__ void k_scale_M_real(DevTables t, const double2 *M, const double4 *cell_x, long long ncells, int P,
-                               float *Msr, unsigned short *Msb) {
+                               float *Msr, unsigned short *Msb, double *Msd) {
   const int NT = t.nterm, ND = nd_of(P), NDP = ndp_of(P);
   const long long total = ncells * NDP;
   for (long long i = blockIdx.x * (long long)blockDim.x + threadIdx.x; i < total; i += (long long)gridDim.x * blockDim.x) {
@@ -309,6 +325,7 @@ __global__ void k_scale_M_real(DevTables t, const double2 *M, const double4 *cel
       v = (part == 0 ? mv.x : mv.y) * s;
     }
     if (Msr) Msr[i] = (float)v;
+    if (Msd) Msd[i] = v;
     if (Msb) {
       unsigned short h[3];
       split_bf16x3(v, h);
@@ -1033,6 +1050,130 @@ k_m2l_class_mma_tma(const __grid_constant__ CUtensorMap msb_map, const int4 *chu
   }
 }
 
+// 6''. The plain method's products, FP64.  Bound: the FP64 pipe (ND^2
+// multiply-adds a pair: 4,096 at P = 8, where the pair-by-pair contraction
+// takes 9,216 and its recurrences).  Persistent blocks of 256 threads take
+// contiguous ranges of chunks, so the operator (ND x NDP, at most 90 KB) stays
+// in shared memory across a class's chunks.  Up to P = 8 a tile is a chunk of
+// 128 pairs and two blocks share an SM, one gathering (cp.async) while the
+// other multiplies; at P = 10 one block holds the operator and two tiles of 64
+// pairs, the next one gathered ahead.  Thread (tx, ty) holds outputs tx + 16 j
+// of pairs ty + 16 v: two inputs of a pair come in one 16-byte read, an operator
+// row is read by 16 consecutive threads, and a pair's outputs are stored in
+// 128-byte runs.  Each output is
+// one FP64 sum over the inputs in order, whatever the chunk, so a pair's
+// contribution does not depend on the pairs beside it.  M2L phase, pair by pair
+// against products: 1M-body Plummer sphere at P = 8 (15.1M pairs) 31.4 -> 11.7
+// ms, of which these products 8.0 (42 % of the FP64 pipe); 100K-body cube at
+// P = 10 (0.6M pairs, about 90 a class) 3.27 -> 2.81 ms.
+__host__ __device__ constexpr int gemm64_rows(int NDP) { return NDP > 64 ? 64 : 128; }
+__host__ __device__ constexpr int gemm64_bufs(int NDP) { return NDP > 64 ? 2 : 1; }
+__host__ __device__ constexpr size_t gemm64_smem_bytes(int NDP, int ND) {
+  return ((size_t)ND * NDP + (size_t)gemm64_bufs(NDP) * gemm64_rows(NDP) * (NDP + 2)) * sizeof(double);
+}
+
+// NV x NJ outputs a thread (pairs ty + 16 v, outputs tx + 16 j) over ND inputs.
+template <int NDP, int NV>
+__device__ __forceinline__ void gemm64_tile(const double *a, const double *b, int ND, const int *q, double *Y, int tx) {
+  constexpr int NJ = NDP / 16, ASTR = NDP + 2;
+  double acc[NV][NJ];
+#pragma unroll
+  for (int v = 0; v < NV; v++)
+#pragma unroll
+    for (int j = 0; j < NJ; j++) acc[v][j] = 0.0;
+#pragma unroll 2
+  for (int k = 0; k < ND; k += 2) {
+    double2 x[NV];
+#pragma unroll
+    for (int v = 0; v < NV; v++) x[v] = *reinterpret_cast<const double2 *>(a + 16 * v * ASTR + k);
+    const double *bk = b + k * NDP + tx;
+#pragma unroll
+    for (int j = 0; j < NJ; j++) {
+      const double b0 = bk[16 * j], b1 = bk[NDP + 16 * j];
+#pragma unroll
+      for (int v = 0; v < NV; v++) acc[v][j] = fma(x[v].y, b1, fma(x[v].x, b0, acc[v][j]));
+    }
+  }
+#pragma unroll
+  for (int v = 0; v < NV; v++) {
+    const int at = q[16 * v];
+    if (at >= 0) {
+#pragma unroll
+      for (int j = 0; j < NJ; j++) Y[(long long)at * NDP + tx + 16 * j] = acc[v][j];
+    }
+  }
+}
+
+template <int NDP>
+__global__ void __launch_bounds__(256, NDP > 64 ? 1 : 2)
+k_m2l_class_gemm64(const int4 *chunks, const int *nchunks, const int *sval, const int *ssrc, const double *K,
+                   const double *Ms, double *Y, int ND) {
+  constexpr int ASTR = NDP + 2, ROWS = gemm64_rows(NDP), BUFS = gemm64_bufs(NDP), PARTS = kChunk / ROWS;
+  constexpr int TPR = 256 / ROWS;  // threads that gather one row
+  extern __shared__ __align__(16) double smem_d[];
+  __shared__ int s_q[2][ROWS];
+  double *sK = smem_d;                      // [input][output]
+  double *sA = smem_d + (size_t)ND * NDP;   // [buffer][pair][input]
+  const int total = *nchunks;
+  const int j0 = (int)((long long)total * blockIdx.x / gridDim.x);
+  const int j1 = (int)((long long)total * (blockIdx.x + 1) / gridDim.x);
+  if (j0 >= j1) return;
+  const int tx = threadIdx.x & 15, ty = threadIdx.x >> 4;
+  const int row = threadIdx.x / TPR, part = threadIdx.x % TPR;  // this thread's share of a gather
+  // tile i of the range: chunk j0 + i / PARTS, its pairs from (i % PARTS) * ROWS on (perhaps none)
+  const int tiles = PARTS * (j1 - j0);
+  auto source = [&](int i, int &q) {
+    q = -1;
+    if (i >= tiles) return -1;
+    const int4 ch = chunks[j0 + i / PARTS];
+    const int at = (i % PARTS) * ROWS + row;
+    if (at >= ch.z) return -1;
+    q = sval[ch.y + at];
+    return ssrc[ch.y + at];
+  };
+  auto gather = [&](int i, int src, int q) {
+    if (part == 0) s_q[i & 1][row] = q;
+    if (src >= 0) {
+      const double *from = Ms + (long long)src * NDP;
+      double *to = sA + (i % BUFS) * ROWS * ASTR + row * ASTR;
+      for (int u = part; u < ND / 2; u += TPR) cp_async16(to + 2 * u, from + 2 * u);
+    }
+    cp_async_commit();
+  };
+  int cur = -1, nq;
+  int next = source(0, nq);
+  if (BUFS == 2) {
+    gather(0, next, nq);
+    next = source(1, nq);
+  }
+  for (int i = 0; i < tiles; i++) {
+    const int4 ch = chunks[j0 + i / PARTS];
+    const int cnt = min(ROWS, ch.z - (i % PARTS) * ROWS);
+    gather(i + BUFS - 1, next, nq);  // its buffer was read before the last barrier
+    next = source(i + BUFS, nq);
+    if (ch.x != cur) {  // a new class: its operator (inputs from ND on are padding)
+      const double *Kg = K + (long long)ch.x * NDP * NDP;
+      for (int u = threadIdx.x; u < ND * NDP / 2; u += 256) cp_async16(sK + 2 * u, Kg + 2 * u);
+      cp_async_commit();
+      cur = ch.x;
+      cp_async_wait_all();
+    } else if (BUFS == 2) {
+      asm volatile("cp.async.wait_group 1;" ::: "memory");
+    } else {
+      cp_async_wait_all();
+    }
+    __syncthreads();
+    const double *a = sA + (i % BUFS) * ROWS * ASTR + ty * ASTR;
+    const int *q = s_q[i & 1] + ty;
+    // whole 16-pair rows of the tile only: classes often end in a short one
+    if (cnt > ROWS / 2) gemm64_tile<NDP, ROWS / 16>(a, sK, ND, q, Y, tx);
+    else if (cnt > ROWS / 4) gemm64_tile<NDP, ROWS / 32>(a, sK, ND, q, Y, tx);
+    else if (cnt > 0) gemm64_tile<NDP, ROWS / 64>(a, sK, ND, q, Y, tx);
+    __syncthreads();
+  }
+  cp_async_wait_all();
+}
+
 // 7. Per target cell, in list order: the sum of its taken pairs' columns of
 // Y (FP64), scaled by (-1)^j A_j^k R_t^{-(j+1)}, added to L.  Lane l holds
 // entries VEC l .. VEC l + VEC - 1 of a column (VEC = 4 floats, one 16-byte
@@ -1040,14 +1181,16 @@ k_m2l_class_mma_tma(const __grid_constant__ CUtensorMap msb_map, const int4 *chu
 // together with its taken flags (the rows of pairs not taken hold whatever is
 // there and are dropped by a select, so the loads do not wait for the flags),
 // and the next group's loads are in flight while this one is added.
-template <int NDP>
-__global__ void k_m2l_class_reduce(const int *off, long long ncells, const unsigned char *taken, const float *Y,
+template <int NDP, typename T>
+__global__ void k_m2l_class_reduce(const int *off, long long ncells, const unsigned char *taken, const T *Y,
                                    const double4 *cell_x, DevTables t, int P, double2 *L) {
   constexpr int VEC = NDP > 64 ? 4 : 2;
   constexpr int LANES = NDP / VEC;  // lanes that hold entries
   static_assert(NDP % VEC == 0 && LANES <= 32, "one row per warp-wide load");
-  constexpr int G = 8;
-  using V = typename std::conditional<VEC == 4, float4, float2>::type;
+  constexpr int G = sizeof(T) * VEC > 16 ? 4 : 8;  // rows in flight
+  struct alignas(VEC * sizeof(T) < 16 ? VEC * sizeof(T) : 16) V {
+    T f[VEC];
+  };
   const int lane = threadIdx.x & 31;
   const bool active = lane < LANES;
   const int NT = t.nterm, ND = nd_of(P);
@@ -1057,7 +1200,7 @@ __global__ void k_m2l_class_reduce(const int *off, long long ncells, const unsig
     v = V{};
     if (q < e) {
       tk = taken[q] != 0;
-      if (active) v = reinterpret_cast<const V *>(Y + (long long)q * NDP)[lane];
+      if (active) v = *reinterpret_cast<const V *>(Y + (long long)q * NDP + VEC * lane);
     }
   };
   for (long long c = (long long)blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5); c < ncells; c += warps) {
@@ -1077,9 +1220,8 @@ __global__ void k_m2l_class_reduce(const int *off, long long ncells, const unsig
       for (int i = 0; i < G; i++) {
         if (!tk[i]) continue;
         any = true;
-        const float *f = reinterpret_cast<const float *>(&v[i]);
 #pragma unroll
-        for (int k = 0; k < VEC; k++) acc[k] += (double)f[k];
+        for (int k = 0; k < VEC; k++) acc[k] += (double)v[i].f[k];
       }
 #pragma unroll
       for (int i = 0; i < G; i++) {
@@ -1163,6 +1305,17 @@ void tma_launch(const CUtensorMap &map, M2LGemmBufs &g, const int *sv, long long
   }
 }
 
+template <int NDP>
+void gemm64_launch(M2LGemmBufs &g, const int *sv, long long chunks_max, int ncls, int ND, cudaStream_t st) {
+  const size_t smem = gemm64_smem_bytes(NDP, ND);
+  set_smem(k_m2l_class_gemm64<NDP>, smem);
+  const int per_sm = std::max(1, std::min(2, (int)(233472 / (smem + 2048))));
+  const long long grid = std::min<long long>(chunks_max, (long long)kNumSMs * per_sm);
+  k_m2l_class_gemm64<NDP><<<(unsigned)grid, 256, smem, st>>>(g.chunks.p, g.cbase.p + ncls, sv, g.ssrc.p, g.K64.p,
+                                                             g.Ms64r.p, g.Y64.p, ND);
+  EXA_CHECK_LAUNCH();
+}
+
 }  // namespace
 
 bool m2l_gemm_supported(int P) { return P == 4 || P == 6 || P == 8 || P == 10; }
@@ -1183,10 +1336,34 @@ bool m2l_gemm_worthwhile(int P, long long n_m2l) {
 }
 constexpr long long kMinPairsPerClass = 80;
 
+// The plain method takes the products from this many pairs (0: never), by the
+// pair count of the solve, or of each system of a forest, alone: a pair's
+// contribution does not depend on the pairs beside it, so a system's results
+// are the same bits alone and in a forest.  The class work (hashing, sorting,
+// operators) costs about 0.5 ms; a pair 0.9, 2.1 and 5.4 ns pair by pair at
+// P = 6, 8 and 10, and 0.3, 0.6 and 2 to 3 ns as a product.  The contributions
+// take 8 NDP bytes a pair: solves that would need over 16 GB stay pair by pair.
+long long m2l_gemm64_pairs(int P) { return P == 6 ? 3000000 : P == 8 ? 1000000 : P == 10 ? 400000 : 0; }
+
+bool m2l_gemm64_worthwhile(int P, long long n_m2l) {
+  const long long least = m2l_gemm64_pairs(P);
+  return least > 0 && n_m2l >= least && n_m2l * ndp_of(P) * 8 <= (16LL << 30);
+}
+
 bool m2l_gemm(Context &C, const FmmArgs &a, M2LGemmBufs &g, long long n_m2l, int min_level, int max_dl) {
   const int P = a.P;
   if (!m2l_gemm_supported(P) || a.ncells <= 0 || n_m2l <= 0) return false;
-  if (!g.force && !m2l_gemm_worthwhile(P, n_m2l)) return false;
+  if (!g.force && !(g.fp64 ? m2l_gemm64_worthwhile(P, n_m2l) : m2l_gemm_worthwhile(P, n_m2l))) return false;
+  if (g.fp64) {  // before any work: without room for the contributions the solve stays pair by pair
+    try {
+      g.Y64.ensure(n_m2l * ndp_of(P));
+    } catch (const std::exception &) {
+      cudaGetLastError();
+      return false;
+    }
+  }
+  // level differences a class key holds; the policy's leftover pairs go pair by pair
+  const int key_dl = std::min(max_dl, 15);
   cudaStream_t st = a.stream;
   const DevTables &t = device_tables(P);
   const long long nc = a.ncells;
@@ -1204,8 +1381,10 @@ bool m2l_gemm(Context &C, const FmmArgs &a, M2LGemmBufs &g, long long n_m2l, int
   EXA_CUDA(cudaMemsetAsync(g.hk.p, 0xff, hcap * sizeof(unsigned long long), st));
   EXA_CUDA(cudaMemsetAsync(g.hid.p, 0xff, hcap * sizeof(int), st));
   EXA_CUDA(cudaMemsetAsync(g.cnt.p, 0, 4 * sizeof(int), st));
-  k_pair_class<<<kNumSMs * 8, 256, 0, st>>>(a.m2l_off, a.m2l_src, nc, a.cell_x, a.cell_pl, min_level, max_dl, g.hk.p,
-                                            hcap - 1, g.pair_slot.p);
+  k_pair_class<<<kNumSMs * 8, 256, 0, st>>>(a.m2l_off, a.m2l_src, nc, a.cell_x, a.cell_pl, min_level, key_dl, g.hk.p,
+                                            hcap - 1, g.pair_slot.p,
+                                            g.fp64 && C.tree.nsys ? C.tree.sys_cell.p : nullptr, C.tree.nsys,
+                                            m2l_gemm64_pairs(P));
   EXA_CHECK_LAUNCH();
   const int ccap = (int)std::min<long long>(hcap, (1LL << kClsBits) - 1);
   g.ck.ensure(ccap);
@@ -1219,7 +1398,7 @@ bool m2l_gemm(Context &C, const FmmArgs &a, M2LGemmBufs &g, long long n_m2l, int
   EXA_CUDA(cudaStreamSynchronize(st));
   int ncls = *ncls_h;
   if (ncls <= 0) return false;
-  if (!g.force && n_m2l < kMinPairsPerClass * (long long)ncls) return false;  // too many classes for their pairs
+  if (!g.force && !g.fp64 && n_m2l < kMinPairsPerClass * (long long)ncls) return false;  // too many classes for their pairs
   if (ncls > ccap) ncls = ccap;  // the overflow classes' pairs stay per-pair
   bool alt = radix_sort_u64((uint64_t *)g.ck.p, g.cs.p, (uint64_t *)g.ck_alt.p, g.cs_alt.p, ncls, 0, 64, C.sort,
                             C.err.p, st);
@@ -1227,26 +1406,28 @@ bool m2l_gemm(Context &C, const FmmArgs &a, M2LGemmBufs &g, long long n_m2l, int
   int *cs = alt ? g.cs_alt.p : g.cs.p;
   k_class_ids<<<(ncls + 255) / 256, 256, 0, st>>>(cs, ncls, g.hid.p);
   EXA_CHECK_LAUNCH();
-  const bool tc = g.tensor_cores;
+  const bool tc = g.tensor_cores && !g.fp64;
   // P = 8 on the tensor cores: source pieces gathered by TMA (its tensor map made below).
   // At P = 10 (two 128-byte K-blocks, one CTA per SM either way) the cp.async
   // form is a little faster (M2L 16.4 vs 16.8 ms on a 1M-charge periodic box).
   CUtensorMap msb_map;
   bool use_tma = tc && NDP == 64 && g.tma && encode_tiled() != nullptr;
   if (tc) g.Kb.ensure((long long)ncls * 3 * (use_tma ? tma_kblocks(NDP) * NDP * 64 : NDP * NDP));
+  else if (g.fp64) g.K64.ensure((long long)ncls * NDP * NDP);
   else g.K.ensure((long long)ncls * NDP * NDP);
   {
     const size_t smem = tri(2 * P - 1) * sizeof(double2);
-    float *Kt = tc ? nullptr : g.K.p;
+    float *Kt = tc || g.fp64 ? nullptr : g.K.p;
     unsigned short *Kb = tc ? g.Kb.p : nullptr;
     auto build = [&](auto kernel) {
-      kernel<<<ncls, 256, smem, st>>>(t, ck, P, Kt, Kb, a.cell_x, a.cycle);
+      kernel<<<ncls, 256, smem, st>>>(t, ck, P, Kt, Kb, g.K64.p, a.cell_x, a.cycle);
       EXA_CHECK_LAUNCH();
     };
     switch (NDP) {
 #define EXA_BUILD_K_CASE(N)                                      \
   case N:                                                        \
-    if (!tc) build(k_build_K<N, kKFp32>);                        \
+    if (g.fp64) build(k_build_K<N, kKFp64>);                     \
+    else if (!tc) build(k_build_K<N, kKFp32>);                   \
     else if (use_tma) build(k_build_K<N, kKSwizzled>);           \
     else build(k_build_K<N, kKCore>);                            \
     break;
@@ -1259,11 +1440,12 @@ bool m2l_gemm(Context &C, const FmmArgs &a, M2LGemmBufs &g, long long n_m2l, int
     }
   }
   if (tc) g.Msb.ensure(nc * 3 * NDP);
+  else if (g.fp64) g.Ms64r.ensure(nc * NDP);
   else g.Msr.ensure(nc * NDP);
   if (use_tma && !msb_tensor_map(&msb_map, g.Msb.p, nc, NDP))
     throw std::runtime_error("TMA tensor map of the multipoles");
-  k_scale_M_real<<<kNumSMs * 8, 256, 0, st>>>(t, a.M64, a.cell_x, nc, P, tc ? nullptr : g.Msr.p,
-                                              tc ? g.Msb.p : nullptr);
+  k_scale_M_real<<<kNumSMs * 8, 256, 0, st>>>(t, a.M64, a.cell_x, nc, P, tc || g.fp64 ? nullptr : g.Msr.p,
+                                              tc ? g.Msb.p : nullptr, g.fp64 ? g.Ms64r.p : nullptr);
   EXA_CHECK_LAUNCH();
   // ---- pairs of classes with an operator, sorted by class
   g.taken.ensure(n_m2l);
@@ -1293,7 +1475,7 @@ bool m2l_gemm(Context &C, const FmmArgs &a, M2LGemmBufs &g, long long n_m2l, int
   ChunkScan cs2{g.cstart.p, g.cbase.p, ncls};
   launch_scan<1024, 8>(cs2, nullptr, ncls, ncls, C.scan, C.err.p, st);
   const long long chunks_max = n_m2l / kChunk + ncls + 1;
-  if (tc) {
+  if (tc || g.fp64) {
     g.chunks.ensure(chunks_max);
     g.ssrc.ensure(n_m2l);
     k_chunk_table<<<(ncls + 255) / 256, 256, 0, st>>>(g.cstart.p, g.cbase.p, ncls, g.chunks.p);
@@ -1303,10 +1485,17 @@ bool m2l_gemm(Context &C, const FmmArgs &a, M2LGemmBufs &g, long long n_m2l, int
     EXA_CHECK_LAUNCH();
   }
   // ---- products per class chunk, then per-target sums
-  g.Y.ensure(n_m2l * NDP);
+  if (!g.fp64) g.Y.ensure(n_m2l * NDP);
   switch (NDP) {
 #define EXA_GEMM_CASE(N)                                                                                      \
   case N: {                                                                                                   \
+    if (g.fp64) {                                                                                             \
+      gemm64_launch<N>(g, sv, chunks_max, ncls, nd_of(P), st);                                                \
+      k_m2l_class_reduce<N, double><<<kNumSMs * 8, 256, 0, st>>>(a.m2l_off, nc, g.taken.p, g.Y64.p, a.cell_x, \
+                                                                 t, P, a.L64);                                \
+      EXA_CHECK_LAUNCH();                                                                                     \
+      break;                                                                                                  \
+    }                                                                                                         \
     if (use_tma) {                                                                                            \
       tma_launch<N>(msb_map, g, sv, chunks_max, ncls, C.err.p, st);                                           \
     } else if (tc) {                                                                                          \
@@ -1322,7 +1511,7 @@ bool m2l_gemm(Context &C, const FmmArgs &a, M2LGemmBufs &g, long long n_m2l, int
                                                                    a.m2l_src, g.K.p, g.Msr.p, g.Y.p);         \
     }                                                                                                         \
     EXA_CHECK_LAUNCH();                                                                                       \
-    k_m2l_class_reduce<N><<<kNumSMs * 8, 256, 0, st>>>(a.m2l_off, nc, g.taken.p, g.Y.p, a.cell_x, t, P, a.L64); \
+    k_m2l_class_reduce<N, float><<<kNumSMs * 8, 256, 0, st>>>(a.m2l_off, nc, g.taken.p, g.Y.p, a.cell_x, t, P, a.L64); \
     EXA_CHECK_LAUNCH();                                                                                       \
     break;                                                                                                    \
   }
