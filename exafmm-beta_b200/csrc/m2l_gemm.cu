@@ -1340,9 +1340,11 @@ constexpr long long kMinPairsPerClass = 80;
 // pair count of the solve, or of each system of a forest, alone: a pair's
 // contribution does not depend on the pairs beside it, so a system's results
 // are the same bits alone and in a forest.  The class work (hashing, sorting,
-// operators) costs about 0.5 ms; a pair 0.9, 2.1 and 5.4 ns pair by pair at
-// P = 6, 8 and 10, and 0.3, 0.6 and 2 to 3 ns as a product.  The contributions
-// take 8 NDP bytes a pair: solves that would need over 16 GB stay pair by pair.
+// operators) costs about 0.5 ms on 100K bodies; measured per pair, pair by pair
+// against products, 2.07 and 0.61 ns at P = 8 (1M-body Plummer sphere), 5.4 and
+// 3.1 ns at P = 10 (100K-body cube); at P = 6 the line follows from the
+// operation counts and is not measured.  The contributions take 8 NDP bytes a
+// pair: solves that would need over 16 GB stay pair by pair.
 long long m2l_gemm64_pairs(int P) { return P == 6 ? 3000000 : P == 8 ? 1000000 : P == 10 ? 400000 : 0; }
 
 bool m2l_gemm64_worthwhile(int P, long long n_m2l) {
