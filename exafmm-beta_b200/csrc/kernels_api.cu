@@ -178,12 +178,18 @@ struct Mini {
     cudaStreamDestroy(st);
   }
   template <typename T>
-  T *up(const T *h, size_t n) {
+  T *scratch(size_t n) {
     void *p = nullptr;
     EXA_CUDA(cudaMalloc(&p, (n ? n : 1) * sizeof(T)));
     bufs.push_back(p);
-    if (n && h) EXA_CUDA(cudaMemcpyAsync(p, h, n * sizeof(T), cudaMemcpyHostToDevice, st));
     return (T *)p;
+  }
+  template <typename T>
+  T *up(const T *h, size_t n) {
+    if (n && !h) throw std::runtime_error("null array");
+    T *p = scratch<T>(n);
+    if (n) EXA_CUDA(cudaMemcpyAsync(p, h, n * sizeof(T), cudaMemcpyHostToDevice, st));
+    return p;
   }
   template <typename T>
   void down(T *h, const T *d, size_t n) {
@@ -269,7 +275,7 @@ int exafmm_direct(const double *targets, long long nt, const double *sources, lo
     const double4 *t = m.up((const double4 *)targets, nt);
     const double4 *s = m.up((const double4 *)sources, ns);
     double4 *r = m.up((const double4 *)trg, nt);
-    direct_fp64(t, nt, s, ns, prange, cycle, r, m.st, [&](long long n) { return m.up((const double4 *)nullptr, n); });
+    direct_fp64(t, nt, s, ns, prange, cycle, r, m.st, [&](long long n) { return m.scratch<double4>(n); });
     m.down((double4 *)trg, r, nt);
   });
 }
@@ -282,7 +288,7 @@ int exafmm_direct_range(const double *targets, long long nt, const double *sourc
     const double4 *t = m.up((const double4 *)targets, nt);
     const double4 *s = m.up((const double4 *)sources, ns);
     double4 *r = m.up((const double4 *)trg, nt);
-    direct_fp64(t, nt, s, ns, prange, cycle, r, m.st, [&](long long n) { return m.up((const double4 *)nullptr, n); });
+    direct_fp64(t, nt, s, ns, prange, cycle, r, m.st, [&](long long n) { return m.scratch<double4>(n); });
     m.down((double4 *)trg, r, nt);
   });
 }

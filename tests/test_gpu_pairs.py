@@ -1,6 +1,8 @@
 """Pair kernels on the GPU against the oracle's direct sum: the direct sum at the
 edges of its target blocks and source tiles, and the P2P kernels at the edges of
 their lane groups, segments and divided leaves (a tree of one leaf is P2P alone)."""
+import ctypes
+
 import numpy as np
 import pytest
 
@@ -49,3 +51,18 @@ def test_tiny_distances_keep_their_weight(ex, d):
     """The squared distance down to a subnormal number (1e-310, good to about 1e-14 of itself)."""
     got = ex.direct(np.zeros((1, 4)), np.array([[d, 0.0, 0.0, 1.0], [0.0, 0.0, 0.0, 5.0]]))
     assert abs(got[0, 0] * d - 1.0) < 1e-10
+
+
+@pytest.mark.parametrize("missing", ["targets", "sources", "results"])
+def test_direct_refuses_a_null_array(ex, missing):
+    a = {k: np.ones((300, 4)) for k in ("targets", "sources", "results")}
+    ptr = {k: None if k == missing else v.ctypes.data for k, v in a.items()}
+    t, s, r = (ptr[k] for k in ("targets", "sources", "results"))
+    assert ex.lib().exafmm_direct(t, 300, s, 300, 0, 0.4, 1.0, r) != 0
+    assert ex.lib().exafmm_direct_range(t, 300, s, 300, 0, 1.0, r) != 0
+    cycle = np.ones(3)
+    assert ex.lib().exafmm_direct_cutoff(ctypes.c_void_p(t), ctypes.c_longlong(300), ctypes.c_void_p(s),
+                                         ctypes.c_longlong(300), 0, ctypes.c_void_p(cycle.ctypes.data),
+                                         ctypes.c_double(1.0), ctypes.c_void_p(r)) != 0
+    got = ex.direct(a["targets"], a["sources"])  # the next call is untouched
+    assert np.all(got == 0)
