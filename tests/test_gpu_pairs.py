@@ -66,3 +66,40 @@ def test_direct_refuses_a_null_array(ex, missing):
                                          ctypes.c_double(1.0), ctypes.c_void_p(r)) != 0
     got = ex.direct(a["targets"], a["sources"])  # the next call is untouched
     assert np.all(got == 0)
+
+
+@pytest.mark.parametrize("charge", [np.inf, np.nan])
+def test_coincident_bodies_drop_any_charge(ex, oracle, charge):
+    """A pair at distance zero has no weight whatever its charge: a body whose charge is not
+    finite leaves itself and the bodies at its own point alone."""
+    x = np.random.default_rng(5).uniform(-1, 1, (200, 4))
+    x[3, :3] = x[7, :3]
+    x[90, :3] = x[7, :3]
+    bad = x.copy()
+    bad[7, 3] = charge
+    x[7, 3] = 0.0
+    at, other = [3, 7, 90], 50
+    ref = oracle.direct(x, x)
+    with ex.Fmm(P=4, ncrit=256) as f:  # one leaf: P2P alone
+        f.set_bodies(bad)
+        f.solve()
+        solved = f.results()
+    for got in (ex.direct(bad, bad), solved):
+        assert _rel(got[at], ref[at]) < TOL64
+        assert not np.isfinite(got[other, 0])
+
+
+@pytest.mark.parametrize("ns", [1, 300])
+def test_a_small_charge_very_near_does_not_overflow(ex, ns):
+    """q / r^2 is taken as (q / r) / r / r: 1 / r^2 alone would overflow at this distance."""
+    d, q = 1e-155, 1e-200
+    s = np.zeros((ns, 4))
+    s[0] = [d, 0.0, 0.0, q]
+    t = np.zeros((1, 4))
+    with ex.Fmm(P=4, ncrit=512) as f:
+        f.set_bodies(np.concatenate([t, s[:1], [[1.0, 1.0, 1.0, 0.0]]]))
+        f.solve()
+        solved = f.results()[:1]
+    for got in (ex.direct(t, s), solved):
+        assert abs(got[0, 0] * d / q - 1.0) < 1e-10
+        assert abs(got[0, 1] * d * d / q - 1.0) < 1e-10
