@@ -6,9 +6,9 @@
 // cell centers in units of the target radius and on the level difference:
 //   acc_j^k = sum_{n,m} s(k,m) (R_s/R_t)^n Ms_n^m S'_{j+n}^{m-k}(d / R_t),
 //   L_j^k  += (-1)^j A_j^k R_t^{-(j+1)} acc_j^k,        Ms = A_n^m M_n^m / R_s^n.
-// Every center is the root center plus dyadic multiples of the radii, so
-// d / min(R_s, R_t) is an integer vector: (level difference, that vector) is a
-// class key.  Written over real degrees of freedom (Re of every coefficient,
+// Every center is the root center plus dyadic multiples of the radii, to
+// rounding, so d / min(R_s, R_t) is an integer vector: (level difference, that
+// vector) is a class key.  Written over real degrees of freedom (Re of every coefficient,
 // Im of those with m > 0: 2 NTERM - P of them, 64 at P = 8), a class's map is
 // one ND x ND real matrix K (built once per solve from FP64 harmonics).
 //
@@ -39,8 +39,9 @@
 // weigh about 2^-24, FP32 rounding.  The CUDA-core one (k_m2l_class_gemm) is a
 // plain FP32 product.
 //
-// The plain method takes the same route in FP64 (k_m2l_class_gemm64): every
-// pair, operators, multipoles, products and contributions in FP64.
+// The plain method takes the same route in FP64 (k_m2l_class_gemm64): operators,
+// multipoles, products and contributions in FP64, for the pairs whose centers
+// are at the class's offset to FP64 precision (on_lattice).
 #include <cuda.h>
 #include <cuda_bf16.h>
 
@@ -128,10 +129,25 @@ __device__ __forceinline__ unsigned long long class_key_image(int lt, int dl, in
          ((unsigned long long)(dy + 32768) << 16) | (unsigned long long)(dz + 32768);
 }
 
+// Whether the centers' separation d is k radii (of rmin), k the rounded offset
+// of its class, to within 2^-48 (3.6e-15) of its length.  The tree rounds every
+// center, so it is not exactly: by a few ulp of the coordinates, up to 4e-15 of
+// a cell at the origin but 1e-12 at level 4 of a unit box centered at 1,000.  The
+// bodies' expansions are about the rounded centers, so in FP64 a pair further
+// off than that stays with the pair-by-pair kernel, which takes d itself.
+__device__ __forceinline__ bool on_lattice(const double (&d)[3], const double (&k)[3], double rmin) {
+  const double len = (fabs(k[0]) + fabs(k[1]) + fabs(k[2])) * rmin;
+#pragma unroll
+  for (int i = 0; i < 3; i++)
+    if (fabs(fma(-k[i], rmin, d[i])) > len * 0x1p-48) return false;
+  return true;
+}
+
 // 1. Per pair of the target-grouped list: its class's hash slot, or -1.
 __global__ void k_pair_class(const int *off, const int *src, long long ncells, const double4 *cell_x,
                              const int2 *cell_pl, int min_level, int max_dl, unsigned long long *hk,
-                             long long hmask, int *pair_slot, const int *sys_cell, int nsys, long long min_pairs) {
+                             long long hmask, int *pair_slot, bool exact, const int *sys_cell, int nsys,
+                             long long min_pairs) {
   const int lane = threadIdx.x & 31;
   const long long warps = (long long)gridDim.x * (blockDim.x >> 5);
   for (long long c = (long long)blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5); c < ncells; c += warps) {
@@ -159,11 +175,12 @@ __global__ void k_pair_class(const int *off, const int *src, long long ncells, c
       if (part && lt >= min_level && lt < 32 && dl <= max_dl && dl >= -max_dl) {
         const double4 Xs = cell_x[cj];
         const double rmin = fmin(Xt.w, Xs.w);
-        const double fx = rint((Xt.x - Xs.x) / rmin), fy = rint((Xt.y - Xs.y) / rmin), fz = rint((Xt.z - Xs.z) / rmin);
-        if (fabs(fx) < 32767 && fabs(fy) < 32767 && fabs(fz) < 32767) {
+        const double d[3] = {Xt.x - Xs.x, Xt.y - Xs.y, Xt.z - Xs.z};
+        const double f[3] = {rint(d[0] / rmin), rint(d[1] / rmin), rint(d[2] / rmin)};
+        if (fabs(f[0]) < 32767 && fabs(f[1]) < 32767 && fabs(f[2]) < 32767 && (!exact || on_lattice(d, f, rmin))) {
           const unsigned long long key =
-              img == 13 ? class_key(dl, (long long)fx, (long long)fy, (long long)fz)
-                        : class_key_image(lt, dl, img, (long long)fx, (long long)fy, (long long)fz);
+              img == 13 ? class_key(dl, (long long)f[0], (long long)f[1], (long long)f[2])
+                        : class_key_image(lt, dl, img, (long long)f[0], (long long)f[1], (long long)f[2]);
           long long h = (long long)(mix64(key) & (unsigned long long)hmask);
           for (int p = 0; p < kProbe; p++) {
             // a slot's key, once set, never changes: read it at L2 and CAS only
@@ -1384,7 +1401,7 @@ bool m2l_gemm(Context &C, const FmmArgs &a, M2LGemmBufs &g, long long n_m2l, int
   EXA_CUDA(cudaMemsetAsync(g.hid.p, 0xff, hcap * sizeof(int), st));
   EXA_CUDA(cudaMemsetAsync(g.cnt.p, 0, 4 * sizeof(int), st));
   k_pair_class<<<kNumSMs * 8, 256, 0, st>>>(a.m2l_off, a.m2l_src, nc, a.cell_x, a.cell_pl, min_level, key_dl, g.hk.p,
-                                            hcap - 1, g.pair_slot.p,
+                                            hcap - 1, g.pair_slot.p, g.fp64,
                                             g.fp64 && C.tree.nsys ? C.tree.sys_cell.p : nullptr, C.tree.nsys,
                                             m2l_gemm64_pairs(P));
   EXA_CHECK_LAUNCH();

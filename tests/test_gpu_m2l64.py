@@ -28,3 +28,21 @@ def test_products_equal_the_oracle_and_the_forest(ex, oracle, datasets, P, n, nc
     ref = oracle.solve(x, P=P, theta=0.4, ncrit=ncrit).trg
     for k in (slice(0, 1), slice(1, 4)):
         assert np.linalg.norm(a[:, k] - ref[:, k]) < TOL * np.linalg.norm(ref[:, k])
+
+
+@pytest.mark.parametrize("shift", [0.0, 1e3, 1e6])
+def test_displaced_boxes_keep_the_centers_offset(ex, oracle, datasets, shift):
+    """The tree rounds every cell's center, by an ulp of the coordinates a level; a class's operator
+    stands for pairs at its integer offset only to 2^-48 of the separation, and the others go pair
+    by pair.  Bound: that, times the few degrees that carry the field (a gradient one more), plus
+    FP64 sums in another order (some thousand terms, 2^-53 sqrt(1000) = 4e-15)."""
+    x = datasets.cube(40021, seed=10)
+    x[:, :3] += shift
+    with ex.Fmm(P=10, theta=0.4, ncrit=24, precision=ex.FP64) as f:
+        f.set_bodies(x)
+        f.solve()
+        got = f.results()
+        assert f.info()["n_m2l"] >= 400000
+    ref = oracle.solve(x, P=10, theta=0.4, ncrit=24).trg
+    for k, bound in ((slice(0, 1), 2e-14), (slice(1, 4), 1e-13)):
+        assert np.linalg.norm(got[:, k] - ref[:, k]) < bound * np.linalg.norm(ref[:, k])
