@@ -143,6 +143,7 @@ def lib() -> ctypes.CDLL:
         "exafmm_batch_set_config_table": (_c_int, [_vp, _vp, _c_int]),
         "exafmm_batch_bucket_p2p": (_c_int, [_vp, _vp, _c_int]),
         "exafmm_set_p2p_targets_per_lane": (_c_int, [_vp, _c_int]),
+        "exafmm_set_m2l_workspace": (_c_int, [_vp, _c_ll]),
         "exafmm_displace_bodies": (_c_int, [_vp, _c_double, ctypes.c_ulonglong]),
         "exafmm_get_bodies": (_c_int, [_vp, _vp]),
         "exafmm_get_bodies_device": (_c_int, [_vp, _vp]),
@@ -243,6 +244,10 @@ class Fmm:
     def set_p2p_targets_per_lane(self, tpl: int):
         """Mixed P2P: targets per lane, 0 by leaf size (two or three), or 2 / 3 for every leaf."""
         self._check(lib().exafmm_set_p2p_targets_per_lane(self._h, int(tpl)))
+
+    def set_m2l_workspace(self, nbytes: int):
+        """Device bytes of the plain method's M2L work areas (default 3 * 2^30); results do not depend on it."""
+        self._check(lib().exafmm_set_m2l_workspace(self._h, int(nbytes)))
 
     # ---- solve steps (examples/fmm.cxx:163-179) ----
     def set_sources(self, xyzq=None):

@@ -420,7 +420,6 @@ struct Engine {
         // take the per-class products at any size; pair by pair, FP32 sums over
         // a lane's sources lose more there (1.5e-6 against the plain method on
         // a 36K-charge water box at P = 8, against 6.8e-7 for the products)
-        gemm.fp64 = false;
         gemm.force = C.prm.mixed_gemm == 2 || (C.prm.mixed_gemm == 1 && C.prm.images > 0);
         gemm.tensor_cores = C.prm.mixed_gemm_tc != 0;
         if (C.prm.mixed_gemm && m2l_gemm(C, a, gemm, lists.n_m2l, C.prm.mixed_min_level, C.prm.mixed_max_dl)) {
@@ -444,18 +443,19 @@ struct Engine {
           m2l_fp64(a, C.prm.mixed_min_level, C.prm.mixed_max_dl);
         }
       } else if (m2l_fast_supported(C.prm.P, false)) {
-        FmmArgs left = a;  // the pairs the pair-by-pair kernel takes
-        gemm.fp64 = true;
-        gemm.force = false;
         // periodic solves stay pair by pair: image pairs form classes per level
         // and image, fewer than 80 pairs each on a box of 36,000 charges
-        if (C.prm.images == 0 && m2l_gemm(C, a, gemm, lists.n_m2l, 0, kMaxLevels)) {
-          left.m2l_off = gemm.left_off.p;
-          left.m2l_src = gemm.left_src.p;
+        const long long n_left = C.prm.images == 0 ? m2l_gemm64(C, a, gemm, lists.n_m2l) : lists.n_m2l;
+        if (n_left > 0) {  // the pairs the pair-by-pair kernel takes
+          FmmArgs left = a;
+          if (n_left < lists.n_m2l) {
+            left.m2l_off = gemm.left_off.p;
+            left.m2l_src = gemm.left_src.p;
+          }
+          Ms.ensure(nc * NT * sizeof(double2));
+          scale_multipoles(a, false, Ms.p);
+          m2l_fast(left, false, Ms.p);
         }
-        Ms.ensure(nc * NT * sizeof(double2));
-        scale_multipoles(a, false, Ms.p);
-        m2l_fast(left, false, Ms.p);
       } else {
         m2l_fp64(a);
       }
@@ -856,6 +856,13 @@ int exafmm_set_p2p_targets_per_lane(exafmm_ctx *ctx, int tpl) {
     if (tpl != 0 && tpl != 2 && tpl != 3) throw std::runtime_error("targets per lane: 0 (by leaf size), 2 or 3");
     ctx->E.C.prm.p2p_tpl = tpl;
     ctx->E.lists_ok = false;
+  });
+}
+
+int exafmm_set_m2l_workspace(exafmm_ctx *ctx, long long bytes) {
+  return guarded(ctx, [&] {
+    if (bytes < 1 << 20) throw std::runtime_error("the M2L workspace needs at least 2^20 bytes");
+    ctx->E.C.prm.m2l_work = bytes;
   });
 }
 

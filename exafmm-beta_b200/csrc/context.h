@@ -8,6 +8,10 @@ namespace exafmm_b200 {
 
 enum Precision : int { kFP64 = 0, kMixed = 1 };
 
+// Default bytes of the plain method's class products: a slab's contributions
+// (two thirds) and a batch of operators (one third).
+constexpr long long kM2LWork = 3LL << 30;
+
 struct Params {
   int P = 10;
   double theta = 0.4;
@@ -24,6 +28,7 @@ struct Params {
   int mixed_max_dl = 3;
   int mixed_gemm = 1;     // per-class products for frequent offset classes: 0 off, 1 where they pay, 2 always
   int mixed_gemm_tc = 1;  // ... on the tensor cores (bf16x3), else FP32 on the CUDA cores
+  long long m2l_work = kM2LWork;  // plain method: bytes of the class products' work areas
   int p2p_tpl = 0;        // mixed P2P targets per lane: 0 by leaf size (two or three), 2 or 3 for every leaf
 };
 

@@ -89,16 +89,21 @@ struct M2LGemmBufs {
   DBuf<int> cstart, cbase;            // class ranges, chunk offsets per class
   DBuf<float> Y;                      // per list entry: the pair's contribution (real dofs)
   DBuf<double> K64, Ms64r, Y64;       // the FP64 products' operators, multipoles and contributions
+  DBuf<int4> ranges;                  // systems of a forest that take them
+  DBuf<int2> slabs;                   // slabs of a system's targets
   DBuf<int> cnt;
   DBuf<int> left_cnt, left_off, left_src;
   DBuf<int> comp_cnt, comp_off, comp_src;  // pairs outside the mixed policy (FP64), per target
-  bool fp64 = false;          // FP64 products (plain method), every pair
   bool force = false;         // use the class products whatever the size (parity tests)
   bool tensor_cores = true;   // tcgen05 bf16x3 products, else FP32 on the CUDA cores
   bool tma = true;            // P = 8 on the tensor cores: source pieces gathered by TMA
 };
 bool m2l_gemm_supported(int P);
 bool m2l_gemm(Context &C, const FmmArgs &a, M2LGemmBufs &g, long long n_m2l, int min_level, int max_dl);
+// The plain method's: every pair of the systems they pay for.  Returns the
+// number of pairs left, 0, all n_m2l (g's lists are then not set) or those in
+// left_off / left_src.
+long long m2l_gemm64(Context &C, const FmmArgs &a, M2LGemmBufs &g, long long n_m2l);
 // The pairs outside the mixed policy compacted into g.comp_off / g.comp_src (CSR by target, list order).
 long long m2l_complement(Context &C, const FmmArgs &a, M2LGemmBufs &g, long long n_m2l, int min_level, int max_dl);
 

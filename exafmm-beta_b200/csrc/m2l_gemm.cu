@@ -46,8 +46,9 @@
 #include <cuda_bf16.h>
 
 #include <algorithm>
-#include <type_traits>
 #include <stdexcept>
+#include <type_traits>
+#include <vector>
 
 #include "fmm.h"
 #include "harmonics.cuh"
@@ -58,6 +59,7 @@ namespace {
 
 constexpr unsigned long long kEmpty = ~0ull;
 constexpr int kClsBits = 20;      // class id field of the pair key
+constexpr int kMaxSlabs = 100;    // k_slabs: at most twice this and one
 constexpr int kProbe = 64;        // hash probe limit (a pair that finds no slot stays per-pair)
 
 __host__ __device__ inline int nd_of(int P) { return P * (P + 1) - P; }
@@ -146,8 +148,7 @@ __device__ __forceinline__ bool on_lattice(const double (&d)[3], const double (&
 // 1. Per pair of the target-grouped list: its class's hash slot, or -1.
 __global__ void k_pair_class(const int *off, const int *src, long long ncells, const double4 *cell_x,
                              const int2 *cell_pl, int min_level, int max_dl, unsigned long long *hk,
-                             long long hmask, int *pair_slot, bool exact, const int *sys_cell, int nsys,
-                             long long min_pairs) {
+                             long long hmask, int *pair_slot) {
   const int lane = threadIdx.x & 31;
   const long long warps = (long long)gridDim.x * (blockDim.x >> 5);
   for (long long c = (long long)blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5); c < ncells; c += warps) {
@@ -155,32 +156,20 @@ __global__ void k_pair_class(const int *off, const int *src, long long ncells, c
     if (b == e) continue;
     const double4 Xt = cell_x[c];
     const int lt = cell_pl[c].y;
-    // a forest's system takes part by its own pair count, as its solo solve does
-    bool part = true;
-    if (sys_cell) {
-      int lo = 0, hi = nsys - 1;  // last s with sys_cell[s] <= c
-      while (lo < hi) {
-        const int mid = (lo + hi + 1) >> 1;
-        if (sys_cell[mid] <= c) lo = mid;
-        else hi = mid - 1;
-      }
-      part = off[sys_cell[lo + 1]] - off[sys_cell[lo]] >= min_pairs;
-    }
     for (int q = b + lane; q < e; q += 32) {
       const int packed = src[q];
       const int cj = packed & 0x3ffffff, img = packed >> 26;
       const int ls = cell_pl[cj].y;
       const int dl = ls - lt;
       int slot = -1;
-      if (part && lt >= min_level && lt < 32 && dl <= max_dl && dl >= -max_dl) {
+      if (lt >= min_level && lt < 32 && dl <= max_dl && dl >= -max_dl) {
         const double4 Xs = cell_x[cj];
         const double rmin = fmin(Xt.w, Xs.w);
-        const double d[3] = {Xt.x - Xs.x, Xt.y - Xs.y, Xt.z - Xs.z};
-        const double f[3] = {rint(d[0] / rmin), rint(d[1] / rmin), rint(d[2] / rmin)};
-        if (fabs(f[0]) < 32767 && fabs(f[1]) < 32767 && fabs(f[2]) < 32767 && (!exact || on_lattice(d, f, rmin))) {
+        const double fx = rint((Xt.x - Xs.x) / rmin), fy = rint((Xt.y - Xs.y) / rmin), fz = rint((Xt.z - Xs.z) / rmin);
+        if (fabs(fx) < 32767 && fabs(fy) < 32767 && fabs(fz) < 32767) {
           const unsigned long long key =
-              img == 13 ? class_key(dl, (long long)f[0], (long long)f[1], (long long)f[2])
-                        : class_key_image(lt, dl, img, (long long)f[0], (long long)f[1], (long long)f[2]);
+              img == 13 ? class_key(dl, (long long)fx, (long long)fy, (long long)fz)
+                        : class_key_image(lt, dl, img, (long long)fx, (long long)fy, (long long)fz);
           long long h = (long long)(mix64(key) & (unsigned long long)hmask);
           for (int p = 0; p < kProbe; p++) {
             // a slot's key, once set, never changes: read it at L2 and CAS only
@@ -218,6 +207,92 @@ __global__ void k_class_ids(const int *cs_sorted, int ncls, int *hid) {
   for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < ncls; i += gridDim.x * blockDim.x) hid[cs_sorted[i]] = i;
 }
 
+// 1'. and 2'. of the plain method, for one system's targets [c0, c1) (pairs from
+// qb on): the class's hash slot per pair (or -1), the number of classes in
+// cnt[0] and of pairs that have one in cnt[1].  The table has at least eight slots
+// per class the caller takes (limit): past the limit no class is added, and
+// cnt[0] says so; up to it every class has its slot, whatever the timing.
+__global__ void k_pair_class64(const int *off, const int *src, long long c0, long long c1, int qb,
+                               const double4 *cell_x, const int2 *cell_pl, unsigned long long *hk, long long hmask,
+                               int limit, int *pair_slot, int *cnt) {
+  const int lane = threadIdx.x & 31;
+  const long long warps = (long long)gridDim.x * (blockDim.x >> 5);
+  int taken = 0;
+  for (long long c = c0 + (long long)blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5); c < c1; c += warps) {
+    const int b = off[c], e = off[c + 1];
+    if (b == e) continue;
+    const double4 Xt = cell_x[c];
+    const int lt = cell_pl[c].y;
+    for (int q = b + lane; q < e; q += 32) {
+      const int cj = src[q] & 0x3ffffff;
+      const int dl = cell_pl[cj].y - lt;
+      int slot = -1;
+      if (dl <= 15 && dl >= -15) {  // what a key holds
+        const double4 Xs = cell_x[cj];
+        const double rmin = fmin(Xt.w, Xs.w);
+        const double d[3] = {Xt.x - Xs.x, Xt.y - Xs.y, Xt.z - Xs.z};
+        const double f[3] = {rint(d[0] / rmin), rint(d[1] / rmin), rint(d[2] / rmin)};
+        if (fabs(f[0]) < 32767 && fabs(f[1]) < 32767 && fabs(f[2]) < 32767 && on_lattice(d, f, rmin)) {
+          taken++;
+          const unsigned long long key = class_key(dl, (long long)f[0], (long long)f[1], (long long)f[2]);
+          long long h = (long long)(mix64(key) & (unsigned long long)hmask);
+          for (long long p = 0; p <= hmask; p++) {
+            unsigned long long old = __ldcg(&hk[h]);
+            if (old == kEmpty || (p & 63) == 63) {
+              if (__ldcg(&cnt[0]) > limit) break;
+              if (old == kEmpty) old = atomicCAS(&hk[h], kEmpty, key);
+              if (old == kEmpty) atomicAdd(&cnt[0], 1);
+            }
+            if (old == kEmpty || old == key) {
+              slot = (int)h;
+              break;
+            }
+            h = (h + 1) & hmask;
+          }
+        }
+      }
+      pair_slot[q - qb] = slot;
+    }
+  }
+  for (int o = 16; o > 0; o >>= 1) taken += __shfl_xor_sync(0xffffffffu, taken, o);
+  if (lane == 0 && taken) atomicAdd(&cnt[1], taken);
+}
+
+__global__ void k_class_ids64(const unsigned long long *hk, long long hcap, unsigned long long *ck, int *hid, int *n) {
+  for (long long h = blockIdx.x * (long long)blockDim.x + threadIdx.x; h < hcap; h += (long long)gridDim.x * blockDim.x)
+    if (hk[h] != kEmpty) {
+      const int i = atomicAdd(n, 1);
+      ck[i] = hk[h];
+      hid[h] = i;
+    }
+}
+
+// The systems of a forest with at least min_pairs pairs: first and end cell, first and end pair.
+__global__ void k_sys_ranges(const int *off, const int *sys_cell, int nsys, int min_pairs, int4 *out, int *n) {
+  for (int s = blockIdx.x * blockDim.x + threadIdx.x; s < nsys; s += gridDim.x * blockDim.x) {
+    const int c0 = sys_cell[s], c1 = sys_cell[s + 1];
+    if (off[c1] - off[c0] >= min_pairs) out[atomicAdd(n, 1)] = make_int4(c0, c1, off[c0], off[c1]);
+  }
+}
+
+// Cuts targets [c0, c1) into slabs of at most `rows` pairs (or one target): out[i] = (first cell, first pair) of
+// slab i and, after the last, (c1, off[c1]).  One thread.
+__global__ void k_slabs(const int *off, int c0, int c1, long long rows, int2 *out, int *n) {
+  int k = 0;
+  for (int c = c0; c < c1; k++) {
+    out[k] = make_int2(c, off[c]);
+    int lo = c + 1, hi = c1;  // last end with at most `rows` pairs
+    while (lo < hi) {
+      const int mid = lo + (hi - lo + 1) / 2;
+      if ((long long)off[mid] - off[c] <= rows) lo = mid;
+      else hi = mid - 1;
+    }
+    c = lo;
+  }
+  out[k] = make_int2(c1, off[c1]);
+  *n = k;
+}
+
 // 3. Operator of each class: FP32 k-major, Kt[class][input dof][output dof]
 // (CUDA-core engine), or three bf16 pieces of it per class, each an operand
 // image of NDP output rows x NDP inputs in the core_off layout (tensor cores).
@@ -230,10 +305,12 @@ __global__ void k_class_ids(const int *cs_sorted, int ncls, int *hid) {
 // divisions, not runtime divisions (the build was bound by integer work).
 enum KLayout : int { kKFp32 = 0, kKCore = 1, kKSwizzled = 2, kKFp64 = 3 };
 
+// With cstart (FP64), classes without a pair in it are left out.
 template <int NDP, int LAYOUT>
 __global__ void __launch_bounds__(256)
 k_build_K(DevTables t, const unsigned long long *ck, int P, float *Kt, unsigned short *Kb, double *Kd,
-          const double4 *cell_x, double cycle) {
+          const double4 *cell_x, double cycle, const int *cstart) {
+  if (LAYOUT == kKFp64 && cstart && cstart[blockIdx.x] == cstart[blockIdx.x + 1]) return;
   extern __shared__ double2 S[];  // S'_p^q, q >= 0, at d / R_t
   constexpr int KB = (NDP + 63) / 64;  // 128-byte K-blocks of the swizzled image
   constexpr int IMG = LAYOUT == kKSwizzled ? KB * NDP * 64 : NDP * NDP;
@@ -376,6 +453,27 @@ __global__ void k_gemm_flags(const int *off, const int *src, long long ncells, c
       pval[q] = q;
       if (cls < 0 && policy_pair(lt, cell_pl[src[q] & 0x3ffffff].y, min_level, max_dl)) left++;
     }
+    for (int o = 16; o > 0; o >>= 1) left += __shfl_xor_sync(0xffffffffu, left, o);
+    if (lane == 0) left_cnt[c] = left;
+  }
+}
+
+// The plain method's flags, for pairs [qb, qb + n).
+__global__ void k_gemm_flags64(const int *pair_slot, const int *hid, long long n, unsigned char *taken, unsigned *pkey,
+                               int *pval) {
+  for (long long q = blockIdx.x * (long long)blockDim.x + threadIdx.x; q < n; q += (long long)gridDim.x * blockDim.x) {
+    const int s = pair_slot[q];
+    taken[q] = s >= 0;
+    pkey[q] = s >= 0 ? (unsigned)hid[s] : 0xffffffffu;
+    pval[q] = (int)q;
+  }
+}
+__global__ void k_left_count(const int *off, long long ncells, const unsigned char *taken, int *left_cnt) {
+  const int lane = threadIdx.x & 31;
+  const long long warps = (long long)gridDim.x * (blockDim.x >> 5);
+  for (long long c = (long long)blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5); c < ncells; c += warps) {
+    int left = 0;
+    for (int q = off[c] + lane; q < off[c + 1]; q += 32) left += !taken[q];
     for (int o = 16; o > 0; o >>= 1) left += __shfl_xor_sync(0xffffffffu, left, o);
     if (lane == 0) left_cnt[c] = left;
   }
@@ -1123,17 +1221,17 @@ __device__ __forceinline__ void gemm64_tile(const double *a, const double *b, in
 
 template <int NDP>
 __global__ void __launch_bounds__(256, NDP > 64 ? 1 : 2)
-k_m2l_class_gemm64(const int4 *chunks, const int *nchunks, const int *sval, const int *ssrc, const double *K,
-                   const double *Ms, double *Y, int ND) {
+k_m2l_class_gemm64(const int4 *chunks, const int *first, const int *last, int cls0, const int *sval, const int *ssrc,
+                   const double *K, const double *Ms, double *Y, int ND) {
   constexpr int ASTR = NDP + 2, ROWS = gemm64_rows(NDP), BUFS = gemm64_bufs(NDP), PARTS = kChunk / ROWS;
   constexpr int TPR = 256 / ROWS;  // threads that gather one row
   extern __shared__ __align__(16) double smem_d[];
   __shared__ int s_q[2][ROWS];
   double *sK = smem_d;                      // [input][output]
   double *sA = smem_d + (size_t)ND * NDP;   // [buffer][pair][input]
-  const int total = *nchunks;
-  const int j0 = (int)((long long)total * blockIdx.x / gridDim.x);
-  const int j1 = (int)((long long)total * (blockIdx.x + 1) / gridDim.x);
+  const int total = *last - *first;
+  const int j0 = *first + (int)((long long)total * blockIdx.x / gridDim.x);
+  const int j1 = *first + (int)((long long)total * (blockIdx.x + 1) / gridDim.x);
   if (j0 >= j1) return;
   const int tx = threadIdx.x & 15, ty = threadIdx.x >> 4;
   const int row = threadIdx.x / TPR, part = threadIdx.x % TPR;  // this thread's share of a gather
@@ -1169,7 +1267,7 @@ k_m2l_class_gemm64(const int4 *chunks, const int *nchunks, const int *sval, cons
     gather(i + BUFS - 1, next, nq);  // its buffer was read before the last barrier
     next = source(i + BUFS, nq);
     if (ch.x != cur) {  // a new class: its operator (inputs from ND on are padding)
-      const double *Kg = K + (long long)ch.x * NDP * NDP;
+      const double *Kg = K + (long long)(ch.x - cls0) * NDP * NDP;
       for (int u = threadIdx.x; u < ND * NDP / 2; u += 256) cp_async16(sK + 2 * u, Kg + 2 * u);
       cp_async_commit();
       cur = ch.x;
@@ -1191,16 +1289,17 @@ k_m2l_class_gemm64(const int4 *chunks, const int *nchunks, const int *sval, cons
   cp_async_wait_all();
 }
 
-// 7. Per target cell, in list order: the sum of its taken pairs' columns of
-// Y (FP64), scaled by (-1)^j A_j^k R_t^{-(j+1)}, added to L.  Lane l holds
+// 7. Per target cell of [c0, c1), in list order: the sum of its taken pairs'
+// columns of Y (FP64; row 0 is pair qb), scaled by (-1)^j A_j^k R_t^{-(j+1)},
+// added to L.  Lane l holds
 // entries VEC l .. VEC l + VEC - 1 of a column (VEC = 4 floats, one 16-byte
 // load per lane and pair, for NDP > 64; else 2).  A group's rows are loaded
 // together with its taken flags (the rows of pairs not taken hold whatever is
 // there and are dropped by a select, so the loads do not wait for the flags),
 // and the next group's loads are in flight while this one is added.
 template <int NDP, typename T>
-__global__ void k_m2l_class_reduce(const int *off, long long ncells, const unsigned char *taken, const T *Y,
-                                   const double4 *cell_x, DevTables t, int P, double2 *L) {
+__global__ void k_m2l_class_reduce(const int *off, long long c0, long long c1, const unsigned char *taken, const T *Y,
+                                   int qb, const double4 *cell_x, DevTables t, int P, double2 *L) {
   constexpr int VEC = NDP > 64 ? 4 : 2;
   constexpr int LANES = NDP / VEC;  // lanes that hold entries
   static_assert(NDP % VEC == 0 && LANES <= 32, "one row per warp-wide load");
@@ -1217,10 +1316,10 @@ __global__ void k_m2l_class_reduce(const int *off, long long ncells, const unsig
     v = V{};
     if (q < e) {
       tk = taken[q] != 0;
-      if (active) v = *reinterpret_cast<const V *>(Y + (long long)q * NDP + VEC * lane);
+      if (active) v = *reinterpret_cast<const V *>(Y + (long long)(q - qb) * NDP + VEC * lane);
     }
   };
-  for (long long c = (long long)blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5); c < ncells; c += warps) {
+  for (long long c = c0 + (long long)blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5); c < c1; c += warps) {
     const int b = off[c], e = off[c + 1];
     double acc[VEC];
 #pragma unroll
@@ -1323,14 +1422,25 @@ void tma_launch(const CUtensorMap &map, M2LGemmBufs &g, const int *sv, long long
 }
 
 template <int NDP>
-void gemm64_launch(M2LGemmBufs &g, const int *sv, long long chunks_max, int ncls, int ND, cudaStream_t st) {
+void gemm64_launch(M2LGemmBufs &g, int cls0, int cls1, const int *sv, long long chunks_max, int ND, cudaStream_t st) {
   const size_t smem = gemm64_smem_bytes(NDP, ND);
   set_smem(k_m2l_class_gemm64<NDP>, smem);
   const int per_sm = std::max(1, std::min(2, (int)(233472 / (smem + 2048))));
   const long long grid = std::min<long long>(chunks_max, (long long)kNumSMs * per_sm);
-  k_m2l_class_gemm64<NDP><<<(unsigned)grid, 256, smem, st>>>(g.chunks.p, g.cbase.p + ncls, sv, g.ssrc.p, g.K64.p,
-                                                             g.Ms64r.p, g.Y64.p, ND);
+  k_m2l_class_gemm64<NDP><<<(unsigned)grid, 256, smem, st>>>(g.chunks.p, g.cbase.p + cls0, g.cbase.p + cls1, cls0, sv,
+                                                             g.ssrc.p, g.K64.p, g.Ms64r.p, g.Y64.p, ND);
   EXA_CHECK_LAUNCH();
+}
+
+template <typename T>
+bool try_ensure(DBuf<T> &b, size_t n) {
+  try {
+    b.ensure(n);
+    return true;
+  } catch (const std::exception &) {
+    cudaGetLastError();
+    return false;
+  }
 }
 
 }  // namespace
@@ -1353,36 +1463,10 @@ bool m2l_gemm_worthwhile(int P, long long n_m2l) {
 }
 constexpr long long kMinPairsPerClass = 80;
 
-// The plain method takes the products from this many pairs (0: never), by the
-// pair count of the solve, or of each system of a forest, alone: a pair's
-// contribution does not depend on the pairs beside it, so a system's results
-// are the same bits alone and in a forest.  The class work (hashing, sorting,
-// operators) costs about 0.5 ms on 100K bodies; measured per pair, pair by pair
-// against products, 2.07 and 0.61 ns at P = 8 (1M-body Plummer sphere), 5.4 and
-// 3.1 ns at P = 10 (100K-body cube); at P = 6 the line follows from the
-// operation counts and is not measured.  The contributions take 8 NDP bytes a
-// pair: solves that would need over 16 GB stay pair by pair.
-long long m2l_gemm64_pairs(int P) { return P == 6 ? 3000000 : P == 8 ? 1000000 : P == 10 ? 400000 : 0; }
-
-bool m2l_gemm64_worthwhile(int P, long long n_m2l) {
-  const long long least = m2l_gemm64_pairs(P);
-  return least > 0 && n_m2l >= least && n_m2l * ndp_of(P) * 8 <= (16LL << 30);
-}
-
 bool m2l_gemm(Context &C, const FmmArgs &a, M2LGemmBufs &g, long long n_m2l, int min_level, int max_dl) {
   const int P = a.P;
   if (!m2l_gemm_supported(P) || a.ncells <= 0 || n_m2l <= 0) return false;
-  if (!g.force && !(g.fp64 ? m2l_gemm64_worthwhile(P, n_m2l) : m2l_gemm_worthwhile(P, n_m2l))) return false;
-  if (g.fp64) {  // before any work: without room for the contributions the solve stays pair by pair
-    try {
-      g.Y64.ensure(n_m2l * ndp_of(P));
-    } catch (const std::exception &) {
-      cudaGetLastError();
-      return false;
-    }
-  }
-  // level differences a class key holds; the policy's leftover pairs go pair by pair
-  const int key_dl = std::min(max_dl, 15);
+  if (!g.force && !m2l_gemm_worthwhile(P, n_m2l)) return false;
   cudaStream_t st = a.stream;
   const DevTables &t = device_tables(P);
   const long long nc = a.ncells;
@@ -1400,10 +1484,8 @@ bool m2l_gemm(Context &C, const FmmArgs &a, M2LGemmBufs &g, long long n_m2l, int
   EXA_CUDA(cudaMemsetAsync(g.hk.p, 0xff, hcap * sizeof(unsigned long long), st));
   EXA_CUDA(cudaMemsetAsync(g.hid.p, 0xff, hcap * sizeof(int), st));
   EXA_CUDA(cudaMemsetAsync(g.cnt.p, 0, 4 * sizeof(int), st));
-  k_pair_class<<<kNumSMs * 8, 256, 0, st>>>(a.m2l_off, a.m2l_src, nc, a.cell_x, a.cell_pl, min_level, key_dl, g.hk.p,
-                                            hcap - 1, g.pair_slot.p, g.fp64,
-                                            g.fp64 && C.tree.nsys ? C.tree.sys_cell.p : nullptr, C.tree.nsys,
-                                            m2l_gemm64_pairs(P));
+  k_pair_class<<<kNumSMs * 8, 256, 0, st>>>(a.m2l_off, a.m2l_src, nc, a.cell_x, a.cell_pl, min_level,
+                                            std::min(max_dl, 15), g.hk.p, hcap - 1, g.pair_slot.p);
   EXA_CHECK_LAUNCH();
   const int ccap = (int)std::min<long long>(hcap, (1LL << kClsBits) - 1);
   g.ck.ensure(ccap);
@@ -1417,7 +1499,7 @@ bool m2l_gemm(Context &C, const FmmArgs &a, M2LGemmBufs &g, long long n_m2l, int
   EXA_CUDA(cudaStreamSynchronize(st));
   int ncls = *ncls_h;
   if (ncls <= 0) return false;
-  if (!g.force && !g.fp64 && n_m2l < kMinPairsPerClass * (long long)ncls) return false;  // too many classes for their pairs
+  if (!g.force && n_m2l < kMinPairsPerClass * (long long)ncls) return false;  // too many classes for their pairs
   if (ncls > ccap) ncls = ccap;  // the overflow classes' pairs stay per-pair
   bool alt = radix_sort_u64((uint64_t *)g.ck.p, g.cs.p, (uint64_t *)g.ck_alt.p, g.cs_alt.p, ncls, 0, 64, C.sort,
                             C.err.p, st);
@@ -1425,28 +1507,26 @@ bool m2l_gemm(Context &C, const FmmArgs &a, M2LGemmBufs &g, long long n_m2l, int
   int *cs = alt ? g.cs_alt.p : g.cs.p;
   k_class_ids<<<(ncls + 255) / 256, 256, 0, st>>>(cs, ncls, g.hid.p);
   EXA_CHECK_LAUNCH();
-  const bool tc = g.tensor_cores && !g.fp64;
+  const bool tc = g.tensor_cores;
   // P = 8 on the tensor cores: source pieces gathered by TMA (its tensor map made below).
   // At P = 10 (two 128-byte K-blocks, one CTA per SM either way) the cp.async
   // form is a little faster (M2L 16.4 vs 16.8 ms on a 1M-charge periodic box).
   CUtensorMap msb_map;
   bool use_tma = tc && NDP == 64 && g.tma && encode_tiled() != nullptr;
   if (tc) g.Kb.ensure((long long)ncls * 3 * (use_tma ? tma_kblocks(NDP) * NDP * 64 : NDP * NDP));
-  else if (g.fp64) g.K64.ensure((long long)ncls * NDP * NDP);
   else g.K.ensure((long long)ncls * NDP * NDP);
   {
     const size_t smem = tri(2 * P - 1) * sizeof(double2);
-    float *Kt = tc || g.fp64 ? nullptr : g.K.p;
+    float *Kt = tc ? nullptr : g.K.p;
     unsigned short *Kb = tc ? g.Kb.p : nullptr;
     auto build = [&](auto kernel) {
-      kernel<<<ncls, 256, smem, st>>>(t, ck, P, Kt, Kb, g.K64.p, a.cell_x, a.cycle);
+      kernel<<<ncls, 256, smem, st>>>(t, ck, P, Kt, Kb, nullptr, a.cell_x, a.cycle, nullptr);
       EXA_CHECK_LAUNCH();
     };
     switch (NDP) {
 #define EXA_BUILD_K_CASE(N)                                      \
   case N:                                                        \
-    if (g.fp64) build(k_build_K<N, kKFp64>);                     \
-    else if (!tc) build(k_build_K<N, kKFp32>);                   \
+    if (!tc) build(k_build_K<N, kKFp32>);                   \
     else if (use_tma) build(k_build_K<N, kKSwizzled>);           \
     else build(k_build_K<N, kKCore>);                            \
     break;
@@ -1459,12 +1539,11 @@ bool m2l_gemm(Context &C, const FmmArgs &a, M2LGemmBufs &g, long long n_m2l, int
     }
   }
   if (tc) g.Msb.ensure(nc * 3 * NDP);
-  else if (g.fp64) g.Ms64r.ensure(nc * NDP);
   else g.Msr.ensure(nc * NDP);
   if (use_tma && !msb_tensor_map(&msb_map, g.Msb.p, nc, NDP))
     throw std::runtime_error("TMA tensor map of the multipoles");
-  k_scale_M_real<<<kNumSMs * 8, 256, 0, st>>>(t, a.M64, a.cell_x, nc, P, tc || g.fp64 ? nullptr : g.Msr.p,
-                                              tc ? g.Msb.p : nullptr, g.fp64 ? g.Ms64r.p : nullptr);
+  k_scale_M_real<<<kNumSMs * 8, 256, 0, st>>>(t, a.M64, a.cell_x, nc, P, tc ? nullptr : g.Msr.p,
+                                              tc ? g.Msb.p : nullptr, nullptr);
   EXA_CHECK_LAUNCH();
   // ---- pairs of classes with an operator, sorted by class
   g.taken.ensure(n_m2l);
@@ -1494,7 +1573,7 @@ bool m2l_gemm(Context &C, const FmmArgs &a, M2LGemmBufs &g, long long n_m2l, int
   ChunkScan cs2{g.cstart.p, g.cbase.p, ncls};
   launch_scan<1024, 8>(cs2, nullptr, ncls, ncls, C.scan, C.err.p, st);
   const long long chunks_max = n_m2l / kChunk + ncls + 1;
-  if (tc || g.fp64) {
+  if (tc) {
     g.chunks.ensure(chunks_max);
     g.ssrc.ensure(n_m2l);
     k_chunk_table<<<(ncls + 255) / 256, 256, 0, st>>>(g.cstart.p, g.cbase.p, ncls, g.chunks.p);
@@ -1504,17 +1583,10 @@ bool m2l_gemm(Context &C, const FmmArgs &a, M2LGemmBufs &g, long long n_m2l, int
     EXA_CHECK_LAUNCH();
   }
   // ---- products per class chunk, then per-target sums
-  if (!g.fp64) g.Y.ensure(n_m2l * NDP);
+  g.Y.ensure(n_m2l * NDP);
   switch (NDP) {
 #define EXA_GEMM_CASE(N)                                                                                      \
   case N: {                                                                                                   \
-    if (g.fp64) {                                                                                             \
-      gemm64_launch<N>(g, sv, chunks_max, ncls, nd_of(P), st);                                                \
-      k_m2l_class_reduce<N, double><<<kNumSMs * 8, 256, 0, st>>>(a.m2l_off, nc, g.taken.p, g.Y64.p, a.cell_x, \
-                                                                 t, P, a.L64);                                \
-      EXA_CHECK_LAUNCH();                                                                                     \
-      break;                                                                                                  \
-    }                                                                                                         \
     if (use_tma) {                                                                                            \
       tma_launch<N>(msb_map, g, sv, chunks_max, ncls, C.err.p, st);                                           \
     } else if (tc) {                                                                                          \
@@ -1530,7 +1602,8 @@ bool m2l_gemm(Context &C, const FmmArgs &a, M2LGemmBufs &g, long long n_m2l, int
                                                                    a.m2l_src, g.K.p, g.Msr.p, g.Y.p);         \
     }                                                                                                         \
     EXA_CHECK_LAUNCH();                                                                                       \
-    k_m2l_class_reduce<N, float><<<kNumSMs * 8, 256, 0, st>>>(a.m2l_off, nc, g.taken.p, g.Y.p, a.cell_x, t, P, a.L64); \
+    k_m2l_class_reduce<N, float><<<kNumSMs * 8, 256, 0, st>>>(a.m2l_off, 0, nc, g.taken.p, g.Y.p, 0, a.cell_x, t,  \
+                                                              P, a.L64);                                      \
     EXA_CHECK_LAUNCH();                                                                                       \
     break;                                                                                                    \
   }
@@ -1544,6 +1617,178 @@ bool m2l_gemm(Context &C, const FmmArgs &a, M2LGemmBufs &g, long long n_m2l, int
   return true;
 }
 
+// The plain method takes the products from this many pairs (0: never), by the
+// pair count of a solve's or a forest's system alone, and every system goes by
+// itself: a pair's contribution does not depend on the pairs beside it, nor on
+// how the targets are cut into slabs, so a system's results are the same bits
+// alone and in a forest.  The class work (hashing, sorting,
+// operators) costs about 0.5 ms on 100K bodies; measured per pair, pair by pair
+// against products, 2.07 and 0.61 ns at P = 8 (1M-body Plummer sphere), 5.4 and
+// 3.1 ns at P = 10 (100K-body cube); at P = 6 the line follows from the
+// operation counts and is not measured.
+long long m2l_gemm64_pairs(int P) { return P == 6 ? 3000000 : P == 8 ? 1000000 : P == 10 ? 400000 : 0; }
+
+namespace {
+
+// One system's pairs (targets [c0, c1), pairs [b, e)) through the class
+// products.  Returns the pairs taken (0: none, and nothing was added).
+long long m2l_gemm64_system(Context &C, const FmmArgs &a, M2LGemmBufs &g, int4 sys) {
+  const int P = a.P, NDP = ndp_of(P), c0 = sys.x, c1 = sys.y, qb0 = sys.z;
+  const long long np = (long long)sys.w - qb0;
+  cudaStream_t st = a.stream;
+  const DevTables &t = device_tables(P);
+  // ---- classes
+  const int limit = (int)(np / 16);  // classes of at least 16 pairs on average
+  long long hcap = 1 << 14;
+  while (hcap < 8LL * limit) hcap <<= 1;
+  g.hk.ensure(hcap);
+  g.hid.ensure(hcap);
+  g.pair_slot.ensure(np);
+  EXA_CUDA(cudaMemsetAsync(g.hk.p, 0xff, hcap * sizeof(unsigned long long), st));
+  EXA_CUDA(cudaMemsetAsync(g.cnt.p, 0, 4 * sizeof(int), st));
+  k_pair_class64<<<kNumSMs * 8, 256, 0, st>>>(a.m2l_off, a.m2l_src, c0, c1, qb0, a.cell_x, a.cell_pl, g.hk.p, hcap - 1,
+                                              limit, g.pair_slot.p, g.cnt.p);
+  EXA_CHECK_LAUNCH();
+  // ---- slabs of whole targets, whose contributions fit the buffer; the
+  // fewer where memory is short
+  long long rows = std::min(np, std::max<long long>(np / kMaxSlabs + 1, C.prm.m2l_work * 2 / 3 / (8LL * NDP)));
+  while (!try_ensure(g.Y64, rows * NDP)) {
+    if (rows <= np / kMaxSlabs + 1) throw std::runtime_error("no device memory for the M2L contributions");
+    rows = std::max(rows / 2, np / kMaxSlabs + 1);
+  }
+  int2 *slab = reinterpret_cast<int2 *>(C.pin + kPinScratch) + 2;  // after the counts
+  int *cnt = reinterpret_cast<int *>(C.pin + kPinScratch);
+  int nslab = 1;
+  slab[0] = make_int2(c0, qb0);
+  slab[1] = make_int2(c1, sys.w);
+  if (rows < np) {
+    g.slabs.ensure(2 * kMaxSlabs + 2);
+    k_slabs<<<1, 1, 0, st>>>(a.m2l_off, c0, c1, rows, g.slabs.p, g.cnt.p + 3);
+    EXA_CHECK_LAUNCH();
+    EXA_CUDA(cudaMemcpyAsync(slab, g.slabs.p, (2 * kMaxSlabs + 2) * sizeof(int2), cudaMemcpyDeviceToHost, st));
+  }
+  EXA_CUDA(cudaMemcpyAsync(cnt, g.cnt.p, 4 * sizeof(int), cudaMemcpyDeviceToHost, st));
+  EXA_CUDA(cudaStreamSynchronize(st));
+  const int ncls = cnt[0];
+  const long long taken = cnt[1];
+  if (rows < np) nslab = cnt[3];
+  if (ncls <= 0 || ncls > limit) return 0;
+  const std::vector<int2> cut(slab, slab + nslab + 1);
+  long long most = 0;
+  for (int i = 0; i < nslab; i++) most = std::max<long long>(most, cut[i + 1].y - cut[i].y);
+  g.Y64.ensure(most * NDP);  // a target with more pairs than that is a slab of its own
+  g.ck.ensure(ncls);
+  k_class_ids64<<<kNumSMs * 4, 256, 0, st>>>(g.hk.p, hcap, g.ck.p, g.hid.p, g.cnt.p + 2);
+  EXA_CHECK_LAUNCH();
+  // ---- operators and multipoles
+  const size_t smem_k = tri(2 * P - 1) * sizeof(double2);
+  auto build = [&](int k0, int k1, const int *cstart) {
+    auto launch = [&](auto kernel) {
+      kernel<<<k1 - k0, 256, smem_k, st>>>(t, g.ck.p + k0, P, nullptr, nullptr, g.K64.p, a.cell_x, a.cycle, cstart);
+      EXA_CHECK_LAUNCH();
+    };
+    if (NDP == 48) launch(k_build_K<48, kKFp64>);
+    else if (NDP == 64) launch(k_build_K<64, kKFp64>);
+    else launch(k_build_K<112, kKFp64>);
+  };
+  g.K64.ensure((long long)ncls * NDP * NDP);
+  build(0, ncls, nullptr);
+  g.Ms64r.ensure(a.ncells * NDP);
+  k_scale_M_real<<<kNumSMs * 8, 256, 0, st>>>(t, a.M64 + (long long)c0 * t.nterm, a.cell_x + c0, c1 - c0, P, nullptr,
+                                              nullptr, g.Ms64r.p + (long long)c0 * NDP);
+  EXA_CHECK_LAUNCH();
+  // ---- per slab: pairs sorted by class, products per class chunk, per-target sums
+  const int end_bit = std::min(32, bits_for(ncls + 1));
+  g.skey.ensure(most);
+  g.skey_alt.ensure(most);
+  g.pval.ensure(most);
+  g.pval_alt.ensure(most);
+  g.ssrc.ensure(most);
+  g.cstart.ensure(ncls + 1);
+  g.cbase.ensure(ncls + 1);
+  g.chunks.ensure(most / kChunk + ncls + 1);
+  for (int i = 0; i < nslab; i++) {
+    const int qb = cut[i].y;
+    const long long n = cut[i + 1].y - qb;
+    if (n <= 0) continue;
+    const int grid = (int)std::min<long long>(kNumSMs * 8, (n + 255) / 256);
+    k_gemm_flags64<<<grid, 256, 0, st>>>(g.pair_slot.p + (qb - qb0), g.hid.p, n, g.taken.p + qb, g.skey.p, g.pval.p);
+    EXA_CHECK_LAUNCH();
+    const bool alt = radix_sort_u32(g.skey.p, g.pval.p, g.skey_alt.p, g.pval_alt.p, n, 0, end_bit, C.sort, C.err.p, st);
+    const unsigned *sk = alt ? g.skey_alt.p : g.skey.p;
+    const int *sv = alt ? g.pval_alt.p : g.pval.p;
+    k_class_ranges<<<(ncls + 256) / 256, 256, 0, st>>>(sk, n, ncls, g.cstart.p);
+    EXA_CHECK_LAUNCH();
+    ChunkScan scan{g.cstart.p, g.cbase.p, ncls};
+    launch_scan<1024, 8>(scan, nullptr, ncls, ncls, C.scan, C.err.p, st);
+    k_chunk_table<<<(ncls + 255) / 256, 256, 0, st>>>(g.cstart.p, g.cbase.p, ncls, g.chunks.p);
+    EXA_CHECK_LAUNCH();
+    k_sorted_sources<<<grid, 256, 0, st>>>(sv, a.m2l_src + qb, g.cstart.p + ncls, g.ssrc.p);
+    EXA_CHECK_LAUNCH();
+    const long long chunks_max = n / kChunk + ncls + 1;
+    auto products = [&](int k0, int k1) {
+      if (NDP == 48) gemm64_launch<48>(g, k0, k1, sv, chunks_max, nd_of(P), st);
+      else if (NDP == 64) gemm64_launch<64>(g, k0, k1, sv, chunks_max, nd_of(P), st);
+      else gemm64_launch<112>(g, k0, k1, sv, chunks_max, nd_of(P), st);
+    };
+    products(0, ncls);
+    auto reduce = [&](auto kernel) {
+      kernel<<<kNumSMs * 8, 256, 0, st>>>(a.m2l_off, cut[i].x, cut[i + 1].x, g.taken.p, g.Y64.p, qb, a.cell_x, t, P,
+                                          a.L64);
+      EXA_CHECK_LAUNCH();
+    };
+    if (NDP == 48) reduce(k_m2l_class_reduce<48, double>);
+    else if (NDP == 64) reduce(k_m2l_class_reduce<64, double>);
+    else reduce(k_m2l_class_reduce<112, double>);
+  }
+  return taken;
+}
+
+}  // namespace
+
+long long m2l_gemm64(Context &C, const FmmArgs &a, M2LGemmBufs &g, long long n_m2l) {
+  const long long least = m2l_gemm64_pairs(a.P), nc = a.ncells;
+  if (least <= 0 || n_m2l < least || nc <= 0) return n_m2l;
+  cudaStream_t st = a.stream;
+  g.cnt.ensure(4);
+  std::vector<int4> systems;
+  if (!a.nsys) {
+    systems.push_back(make_int4(0, (int)nc, 0, (int)n_m2l));
+  } else {
+    const int cap = (int)std::min<long long>(a.nsys, n_m2l / least);
+    g.ranges.ensure(cap);
+    EXA_CUDA(cudaMemsetAsync(g.cnt.p, 0, sizeof(int), st));
+    k_sys_ranges<<<std::min(kNumSMs, div_up(a.nsys, 128)), 128, 0, st>>>(a.m2l_off, C.tree.sys_cell.p, a.nsys,
+                                                                         (int)least, g.ranges.p, g.cnt.p);
+    EXA_CHECK_LAUNCH();
+    int *n = reinterpret_cast<int *>(C.pin + kPinScratch);
+    EXA_CUDA(cudaMemcpyAsync(n, g.cnt.p, sizeof(int), cudaMemcpyDeviceToHost, st));
+    EXA_CUDA(cudaStreamSynchronize(st));
+    systems.resize(*n);
+    if (*n > 0) {
+      EXA_CUDA(cudaMemcpyAsync(systems.data(), g.ranges.p, *n * sizeof(int4), cudaMemcpyDeviceToHost, st));
+      EXA_CUDA(cudaStreamSynchronize(st));
+    }
+  }
+  if (systems.empty()) return n_m2l;
+  g.taken.ensure(n_m2l);
+  EXA_CUDA(cudaMemsetAsync(g.taken.p, 0, n_m2l, st));
+  long long left = n_m2l;
+  for (const int4 &sys : systems) left -= m2l_gemm64_system(C, a, g, sys);
+  if (left == 0 || left == n_m2l) return left;
+  g.left_cnt.ensure(nc);
+  g.left_off.ensure(nc + 1);
+  g.left_src.ensure(left);
+  const int grid = (int)std::min<long long>(kNumSMs * 8, (nc + 7) / 8);
+  k_left_count<<<grid, 256, 0, st>>>(a.m2l_off, nc, g.taken.p, g.left_cnt.p);
+  EXA_CHECK_LAUNCH();
+  LeftScan ls{g.left_cnt.p, g.left_off.p, nc};
+  launch_scan<1024, 8>(ls, nullptr, nc, nc, C.scan, C.err.p, st);
+  k_left_fill<<<grid, 256, 0, st>>>(a.m2l_off, a.m2l_src, nc, g.taken.p, a.cell_pl, 0, kMaxLevels, g.left_off.p,
+                                    g.left_src.p);
+  EXA_CHECK_LAUNCH();
+  return left;
+}
 long long m2l_complement(Context &C, const FmmArgs &a, M2LGemmBufs &g, long long n_m2l, int min_level, int max_dl) {
   const long long nc = a.ncells;
   cudaStream_t st = a.stream;

@@ -74,6 +74,10 @@ int exafmm_set_mixed_policy(exafmm_ctx *ctx, int m2l_fp32, int p2p_fp32, int min
  * bar either way, though their bits differ.  No counterpart in the reference
  * (its P2P is a SIMD loop over targets, kernels/laplace.h:150-235). */
 int exafmm_set_p2p_targets_per_lane(exafmm_ctx *ctx, int tpl);
+/* Plain method: device bytes that the work areas of a large solve's M2L (its
+ * per-class products) may take, at least 2^20; default 3 * 2^30.  A larger
+ * solve goes through them in pieces; the results do not depend on it. */
+int exafmm_set_m2l_workspace(exafmm_ctx *ctx, long long bytes);
 
 /* Separate source bodies (examples/fmm.cxx -j IneJ, :37-47, :61-73): the next
  * solves evaluate the field of these n sources (n x 4: x, y, z, q, caller

@@ -46,3 +46,41 @@ def test_displaced_boxes_keep_the_centers_offset(ex, oracle, datasets, shift):
     ref = oracle.solve(x, P=10, theta=0.4, ncrit=24).trg
     for k, bound in ((slice(0, 1), 2e-14), (slice(1, 4), 1e-13)):
         assert np.linalg.norm(got[:, k] - ref[:, k]) < bound * np.linalg.norm(ref[:, k])
+
+
+def test_a_large_forest_keeps_every_systems_bits(ex, datasets):
+    """Whether a system takes the products goes by its own pairs alone: here the forest's
+    contributions would be 18 GB together."""
+    x = datasets.cube(40021, seed=10)
+    kw = dict(P=10, theta=0.4, ncrit=24, precision=ex.FP64)
+    with ex.Fmm(**kw) as f:
+        f.set_bodies(x)
+        f.solve()
+        solo = f.results()
+        pairs = f.info()["n_m2l"]
+    assert pairs >= 400000
+    count = int(18e9 / (8 * 112 * pairs)) + 1
+    with ex.Fmm(**kw) as f:
+        f.set_systems([x] * count)
+        f.solve()
+        assert f.info()["n_m2l"] == count * pairs
+        for r in f.system_results():
+            assert np.array_equal(r, solo)
+
+
+@pytest.mark.parametrize("P,n,ncrit,dist", [(6, 90007, 8, "cube"), (8, 60013, 16, "plummer"), (10, 40021, 24, "cube")])
+def test_the_workspace_changes_no_bit(ex, datasets, P, n, ncrit, dist):
+    x = getattr(datasets, dist)(n, seed=P)
+    kw = dict(P=P, theta=0.4, ncrit=ncrit, precision=ex.FP64)
+    out = []
+    for work in (None, 200 << 20, 1 << 20):  # one piece, a few, as many as there are
+        with ex.Fmm(**kw) as f:
+            if work:
+                f.set_m2l_workspace(work)
+            f.set_bodies(x)
+            f.solve()
+            out.append((f.results(), f.device_bytes()))
+    assert np.array_equal(out[1][0], out[0][0]) and np.array_equal(out[2][0], out[0][0])
+    assert out[2][1] < out[1][1] < out[0][1]
+    with ex.Fmm(**kw) as f, pytest.raises(ex.FmmError):
+        f.set_m2l_workspace(0)
