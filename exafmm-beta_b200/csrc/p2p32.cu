@@ -232,6 +232,7 @@ __device__ __forceinline__ void p2p_stream(int lS, Stage &sm, P2PState &st, cons
     if (filled == 0) break;
     const int steps = (filled + 2 * G - 1) >> (6 - lS);  // pair steps per group
     const int padded = 2 * G * (steps + (steps & 1));    // even step count for the unrolled loop
+#pragma unroll 1  // as in p2p_fill
     for (int k = filled + lane; k < padded; k += 32) stage_dummy(sm, k);
     __syncwarp();
 

@@ -59,7 +59,7 @@ struct P2PScan {
     const unsigned long long x = (unsigned long long)ns * (unsigned)slots;
     // segments: a rule on this leaf alone
     const unsigned long long c1 = (unsigned)seg_cost;
-    const unsigned long long sc = x > 32 * c1 ? 4 * c1 : min(max(x / 2, c1), 8 * c1);
+    const unsigned long long sc = min(max(x / 2, c1), 8 * c1);
     const int want = max(1, max((int)(sc / slots), ns / kMaxSeg));
     l.seg = (want + kSegAlign - 1) / kSegAlign * kSegAlign;
     l.nseg = (int)(((long long)ns + l.seg - 1) / l.seg);

@@ -7,19 +7,23 @@
 // (FP64) of a P2P phase whose arithmetic fills the GPU for 0.2 or 0.3 ms.  So
 //   * every leaf's source stream (the bodies of its list's leaves, one after
 //     another) is cut into segments by a fixed rule on the leaf alone: a
-//     multiple of kSegAlign sources, in units c of the kernel's segment cost
-//     (target slots x sources) half the leaf within c to 8 c, 4 c for leaves
-//     above 32 c, at most kMaxSeg segments; a leaf's result is the sum of its
-//     segments' sums in order (fewer, longer segments cost less on large trees:
-//     at 4M bodies P2P 18.9 ms with quarters of a leaf, 18.0 with no cuts; the
-//     costly leaves of small trees need the shorter ones to be shared out);
+//     multiple of kSegAlign sources, half the leaf within c to 8 c, in units c of
+//     the kernel's segment cost (target slots x sources), at most kMaxSeg
+//     segments; a leaf's result is the sum of its segments' sums in order.  The
+//     upper end, mixed P2P: 8 c against 4 c for leaves above 32 c takes 4M bodies
+//     from 17.38 to 17.34 ms and a 1M-charge water box from 4.47 to 4.40, at the
+//     same time on a 100,000-body cube, whose costly leaves need their segments
+//     shared out (a quarter of the leaf: 0.55 ms against 0.36; whole leaves 0.83);
 //   * a leaf may be divided into items of whole segments, taken by different
 //     warps; these leave each segment's sums in scratch and the last warp to
 //     finish adds them in order.  A leaf taken whole adds its segments in the
 //     same order, so how leaves are divided (which depends on what else is in
 //     the solve) does not change a bit of the result.  Divided are the leaves
-//     that cost more than a quarter of a resident warp's share, and every
-//     eighth of the others above 1/16 into items of 1/64 of a share;
+//     that cost more than a quarter of a resident warp's share (FP64 P2P of the
+//     100,000-body cube 0.46 ms, 0.52 with half a share), and every
+//     eighth of the others above 1/16 into items of 1/64 of a share, for the end
+//     of the queue (mixed P2P of a 7,019-body sphere 82 us, 87 without; the same
+//     time from 100,000 bodies on);
 //   * items are queued in four classes, those above 1/2, 1/8 and 1/32 of a
 //     share first, so that the persistent warps finish together.
 // Building the queue is two launches (costs, then one scan that emits the
@@ -121,7 +125,6 @@ struct P2PState {
   int at, tb;         // first source of this segment, first target of this pass
   int4 pos;           // place in the stream (q, o, qw), sources left of this segment
   int4 win[32];       // the window's entries: first body, bodies, image
-  double sum[4][96];  // of a whole leaf: the pass's targets over the segments so far
 };
 
 // The window of list entries from q on.
@@ -179,6 +182,9 @@ __device__ __forceinline__ int p2p_fill(P2PState &st, int room, const int *src, 
     }
     const int4 e = st.win[p.x - p.z];
     const int m = min(min(room - filled, e.y - p.y), p.w);
+    // one or two rounds; unrolled, the hot code outgrows the instruction cache
+    // (mixed P2P of 4M bodies 17.73 against 17.54 ms)
+#pragma unroll 1
     for (int k = lane; k < m; k += 32) stage(filled + k, (long long)e.x + p.y + k, e.z);
     filled += m;
     p.w -= m;
@@ -206,19 +212,23 @@ __device__ __forceinline__ void p2p_finish(const P2PItems &w, P2PState &st, doub
   if (old != lf.y - 1) return;
   __threadfence();
   for (int i = threadIdx.x & 31; i < n; i += 32) {
-    double t[4] = {0.0, 0.0, 0.0, 0.0};
+    double4 r = trg[first + i];
     for (int s = 0; s < lf.z; s++) {
       const double *v = reinterpret_cast<const double *>(w.scratch + base + (long long)s * n + i);
-#pragma unroll
-      for (int k = 0; k < 4; k++) t[k] += __ldcg(v + k);
+      r.x += __ldcg(v);
+      r.y -= __ldcg(v + 1);
+      r.z -= __ldcg(v + 2);
+      r.w -= __ldcg(v + 3);
     }
-    p2p_add(trg + first + i, t);
+    trg[first + i] = r;
   }
 }
 
 // The sums of the pass's target j (lane-group member and slot) over one
-// segment: kept for p2p_finish, or added up in shared memory and, after the
-// item's last segment, to the result (both start from zero and add in order).
+// segment: kept for p2p_finish, or added to the result at once (either way
+// segment by segment, in order).  Added up in shared memory instead, they took
+// 3 KB of a warp's 12 and the L1 that this leaves (mixed P2P of 4M bodies 17.54
+// against 17.38 ms).
 __device__ __forceinline__ void p2p_store(const P2PItems &w, P2PState &st, int j, const double (&v)[4],
                                           double4 *trg) {
   const int i = st.tb + j;
@@ -227,15 +237,7 @@ __device__ __forceinline__ void p2p_store(const P2PItems &w, P2PState &st, int j
     w.scratch[st.item.w + (long long)(st.at / st.seg) * st.cb.y + i] = make_double4(v[0], v[1], v[2], v[3]);
     return;
   }
-  double t[4];
-#pragma unroll
-  for (int k = 0; k < 4; k++) t[k] = (st.at == 0 ? 0.0 : st.sum[k][j]) + v[k];
-  if (st.at + st.seg >= st.item.z) {
-    p2p_add(trg + st.cb.x + i, t);
-  } else {
-#pragma unroll
-    for (int k = 0; k < 4; k++) st.sum[k][j] = t[k];
-  }
+  p2p_add(trg + st.cb.x + i, v);
 }
 
 // The item's leaf and list into st.
