@@ -209,7 +209,8 @@ __global__ void k_class_ids(const int *cs_sorted, int ncls, int *hid) {
 
 // 1'. and 2'. of the plain method, for one system's targets [c0, c1) (pairs from
 // qb on): the class's hash slot per pair (or -1), the number of classes in
-// cnt[0] and of pairs that have one in cnt[1].  The table has at least eight slots
+// cnt[0], of pairs that have one in cnt[1] and of the pair-by-pair kernel's
+// steps for these (32 pairs of a target or what is left) in cnt[2].  The table has at least eight slots
 // per class the caller takes (limit): past the limit no class is added, and
 // cnt[0] says so; up to it every class has its slot, whatever the timing.
 __global__ void k_pair_class64(const int *off, const int *src, long long c0, long long c1, int qb,
@@ -217,12 +218,13 @@ __global__ void k_pair_class64(const int *off, const int *src, long long c0, lon
                                int limit, int *pair_slot, int *cnt) {
   const int lane = threadIdx.x & 31;
   const long long warps = (long long)gridDim.x * (blockDim.x >> 5);
-  int taken = 0;
+  int taken = 0, steps = 0;
   for (long long c = c0 + (long long)blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5); c < c1; c += warps) {
     const int b = off[c], e = off[c + 1];
     if (b == e) continue;
     const double4 Xt = cell_x[c];
     const int lt = cell_pl[c].y;
+    int here = 0;
     for (int q = b + lane; q < e; q += 32) {
       const int cj = src[q] & 0x3ffffff;
       const int dl = cell_pl[cj].y - lt;
@@ -233,7 +235,7 @@ __global__ void k_pair_class64(const int *off, const int *src, long long c0, lon
         const double d[3] = {Xt.x - Xs.x, Xt.y - Xs.y, Xt.z - Xs.z};
         const double f[3] = {rint(d[0] / rmin), rint(d[1] / rmin), rint(d[2] / rmin)};
         if (fabs(f[0]) < 32767 && fabs(f[1]) < 32767 && fabs(f[2]) < 32767 && on_lattice(d, f, rmin)) {
-          taken++;
+          here++;
           const unsigned long long key = class_key(dl, (long long)f[0], (long long)f[1], (long long)f[2]);
           long long h = (long long)(mix64(key) & (unsigned long long)hmask);
           for (long long p = 0; p <= hmask; p++) {
@@ -253,9 +255,14 @@ __global__ void k_pair_class64(const int *off, const int *src, long long c0, lon
       }
       pair_slot[q - qb] = slot;
     }
+    for (int o = 16; o > 0; o >>= 1) here += __shfl_xor_sync(0xffffffffu, here, o);
+    taken += here;
+    steps += (here + 31) / 32;
   }
-  for (int o = 16; o > 0; o >>= 1) taken += __shfl_xor_sync(0xffffffffu, taken, o);
-  if (lane == 0 && taken) atomicAdd(&cnt[1], taken);
+  if (lane == 0 && taken) {
+    atomicAdd(&cnt[1], taken);
+    atomicAdd(&cnt[2], steps);
+  }
 }
 
 __global__ void k_class_ids64(const unsigned long long *hk, long long hcap, unsigned long long *ck, int *hid, int *n) {
@@ -1290,8 +1297,7 @@ k_m2l_class_gemm64(const int4 *chunks, const int *first, const int *last, int cl
 }
 
 // 7. Per target cell of [c0, c1), in list order: the sum of its taken pairs'
-// columns of Y (FP64; row 0 is pair qb), scaled by (-1)^j A_j^k R_t^{-(j+1)},
-// added to L.  Lane l holds
+// columns of Y (FP64), scaled by (-1)^j A_j^k R_t^{-(j+1)}, added to L.  Lane l holds
 // entries VEC l .. VEC l + VEC - 1 of a column (VEC = 4 floats, one 16-byte
 // load per lane and pair, for NDP > 64; else 2).  A group's rows are loaded
 // together with its taken flags (the rows of pairs not taken hold whatever is
@@ -1299,7 +1305,7 @@ k_m2l_class_gemm64(const int4 *chunks, const int *first, const int *last, int cl
 // and the next group's loads are in flight while this one is added.
 template <int NDP, typename T>
 __global__ void k_m2l_class_reduce(const int *off, long long c0, long long c1, const unsigned char *taken, const T *Y,
-                                   int qb, const double4 *cell_x, DevTables t, int P, double2 *L) {
+                                   const double4 *cell_x, DevTables t, int P, double2 *L) {
   constexpr int VEC = NDP > 64 ? 4 : 2;
   constexpr int LANES = NDP / VEC;  // lanes that hold entries
   static_assert(NDP % VEC == 0 && LANES <= 32, "one row per warp-wide load");
@@ -1316,7 +1322,7 @@ __global__ void k_m2l_class_reduce(const int *off, long long c0, long long c1, c
     v = V{};
     if (q < e) {
       tk = taken[q] != 0;
-      if (active) v = *reinterpret_cast<const V *>(Y + (long long)(q - qb) * NDP + VEC * lane);
+      if (active) v = *reinterpret_cast<const V *>(Y + (long long)q * NDP + VEC * lane);
     }
   };
   for (long long c = c0 + (long long)blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5); c < c1; c += warps) {
@@ -1602,8 +1608,8 @@ bool m2l_gemm(Context &C, const FmmArgs &a, M2LGemmBufs &g, long long n_m2l, int
                                                                    a.m2l_src, g.K.p, g.Msr.p, g.Y.p);         \
     }                                                                                                         \
     EXA_CHECK_LAUNCH();                                                                                       \
-    k_m2l_class_reduce<N, float><<<kNumSMs * 8, 256, 0, st>>>(a.m2l_off, 0, nc, g.taken.p, g.Y.p, 0, a.cell_x, t,  \
-                                                              P, a.L64);                                      \
+    k_m2l_class_reduce<N, float><<<kNumSMs * 8, 256, 0, st>>>(a.m2l_off, 0, nc, g.taken.p, g.Y.p, a.cell_x, t, P,  \
+                                                              a.L64);                                         \
     EXA_CHECK_LAUNCH();                                                                                       \
     break;                                                                                                    \
   }
@@ -1621,12 +1627,24 @@ bool m2l_gemm(Context &C, const FmmArgs &a, M2LGemmBufs &g, long long n_m2l, int
 // pair count of a solve's or a forest's system alone, and every system goes by
 // itself: a pair's contribution does not depend on the pairs beside it, nor on
 // how the targets are cut into slabs, so a system's results are the same bits
-// alone and in a forest.  The class work (hashing, sorting,
-// operators) costs about 0.5 ms on 100K bodies; measured per pair, pair by pair
-// against products, 2.07 and 0.61 ns at P = 8 (1M-body Plummer sphere), 5.4 and
-// 3.1 ns at P = 10 (100K-body cube); at P = 6 the line follows from the
-// operation counts and is not measured.
+// alone and in a forest.  M2L phase, pair by pair against products: 3.25 and
+// 2.18 ms for 0.6M pairs at P = 10 (100K-body cube), 2.82 and 1.25 for 1.5M at
+// P = 8 (200K-body cube), 2.16 and 1.87 for 3.3M at P = 6 (300K-body Plummer
+// sphere); below the lines the products still won where classes were large (1.67
+// and 0.80 ms for 0.3M at P = 10, 0.99 and 0.57 for 0.3M at P = 8, 0.97 and 0.86
+// for 1.5M at P = 6), but the 0.5 ms of class work weighs more there.
 long long m2l_gemm64_pairs(int P) { return P == 6 ? 3000000 : P == 8 ? 1000000 : P == 10 ? 400000 : 0; }
+
+// And only where the classes, each of which costs an operator, save at least
+// this many pairs' places in the pair-by-pair kernel's steps on average.
+// Products against pair by pair over 62 systems of cubes, spheres, Plummer
+// spheres and clumps of very different widths (30K to 1.5M bodies, theta 0.3 to
+// 0.5): at P = 8 and 10 they lose at 33 (Plummer sphere, 31 pairs a class: 3.81
+// against 2.97 and 10.3 against 7.13 ms), break even at 32 to 36 with half the
+// pairs off the lattice and win from 41 on (clumps: 3.81 against 5.23 and 9.72
+// against 13.0 ms); at P = 6 they lose at 175 (7.07 against 5.19) and win at 430
+// (8.08 against 9.23).
+int m2l_gemm64_places(int P) { return P == 6 ? 320 : 40; }
 
 namespace {
 
@@ -1638,47 +1656,47 @@ long long m2l_gemm64_system(Context &C, const FmmArgs &a, M2LGemmBufs &g, int4 s
   cudaStream_t st = a.stream;
   const DevTables &t = device_tables(P);
   // ---- classes
-  const int limit = (int)(np / 16);  // classes of at least 16 pairs on average
+  const int limit = (int)(np / 16);  // no more classes than that pay in any case
   long long hcap = 1 << 14;
   while (hcap < 8LL * limit) hcap <<= 1;
   g.hk.ensure(hcap);
   g.hid.ensure(hcap);
   g.pair_slot.ensure(np);
   EXA_CUDA(cudaMemsetAsync(g.hk.p, 0xff, hcap * sizeof(unsigned long long), st));
-  EXA_CUDA(cudaMemsetAsync(g.cnt.p, 0, 4 * sizeof(int), st));
+  EXA_CUDA(cudaMemsetAsync(g.cnt.p, 0, 5 * sizeof(int), st));
   k_pair_class64<<<kNumSMs * 8, 256, 0, st>>>(a.m2l_off, a.m2l_src, c0, c1, qb0, a.cell_x, a.cell_pl, g.hk.p, hcap - 1,
                                               limit, g.pair_slot.p, g.cnt.p);
   EXA_CHECK_LAUNCH();
-  // ---- slabs of whole targets, whose contributions fit the buffer; the
-  // fewer where memory is short
+  int *cnt = reinterpret_cast<int *>(C.pin + kPinScratch);
+  EXA_CUDA(cudaMemcpyAsync(cnt, g.cnt.p, 3 * sizeof(int), cudaMemcpyDeviceToHost, st));
+  EXA_CUDA(cudaStreamSynchronize(st));
+  const int ncls = cnt[0];
+  const long long taken = cnt[1];
+  if (ncls <= 0 || ncls > limit || (long long)ncls * m2l_gemm64_places(P) > 32LL * cnt[2]) return 0;
+  // ---- slabs of whole targets, whose contributions fit the buffer; smaller
+  // ones where memory is short
   long long rows = std::min(np, std::max<long long>(np / kMaxSlabs + 1, C.prm.m2l_work * 2 / 3 / (8LL * NDP)));
   while (!try_ensure(g.Y64, rows * NDP)) {
     if (rows <= np / kMaxSlabs + 1) throw std::runtime_error("no device memory for the M2L contributions");
     rows = std::max(rows / 2, np / kMaxSlabs + 1);
   }
-  int2 *slab = reinterpret_cast<int2 *>(C.pin + kPinScratch) + 2;  // after the counts
-  int *cnt = reinterpret_cast<int *>(C.pin + kPinScratch);
-  int nslab = 1;
-  slab[0] = make_int2(c0, qb0);
-  slab[1] = make_int2(c1, sys.w);
+  std::vector<int2> cut{make_int2(c0, qb0), make_int2(c1, sys.w)};
   if (rows < np) {
     g.slabs.ensure(2 * kMaxSlabs + 2);
     k_slabs<<<1, 1, 0, st>>>(a.m2l_off, c0, c1, rows, g.slabs.p, g.cnt.p + 3);
     EXA_CHECK_LAUNCH();
+    int2 *slab = reinterpret_cast<int2 *>(C.pin + kPinScratch) + 1;
     EXA_CUDA(cudaMemcpyAsync(slab, g.slabs.p, (2 * kMaxSlabs + 2) * sizeof(int2), cudaMemcpyDeviceToHost, st));
+    EXA_CUDA(cudaMemcpyAsync(cnt, g.cnt.p + 3, sizeof(int), cudaMemcpyDeviceToHost, st));
+    EXA_CUDA(cudaStreamSynchronize(st));
+    cut.assign(slab, slab + *cnt + 1);
   }
-  EXA_CUDA(cudaMemcpyAsync(cnt, g.cnt.p, 4 * sizeof(int), cudaMemcpyDeviceToHost, st));
-  EXA_CUDA(cudaStreamSynchronize(st));
-  const int ncls = cnt[0];
-  const long long taken = cnt[1];
-  if (rows < np) nslab = cnt[3];
-  if (ncls <= 0 || ncls > limit) return 0;
-  const std::vector<int2> cut(slab, slab + nslab + 1);
+  const int nslab = (int)cut.size() - 1;
   long long most = 0;
   for (int i = 0; i < nslab; i++) most = std::max<long long>(most, cut[i + 1].y - cut[i].y);
   g.Y64.ensure(most * NDP);  // a target with more pairs than that is a slab of its own
   g.ck.ensure(ncls);
-  k_class_ids64<<<kNumSMs * 4, 256, 0, st>>>(g.hk.p, hcap, g.ck.p, g.hid.p, g.cnt.p + 2);
+  k_class_ids64<<<kNumSMs * 4, 256, 0, st>>>(g.hk.p, hcap, g.ck.p, g.hid.p, g.cnt.p + 4);
   EXA_CHECK_LAUNCH();
   // ---- operators and multipoles
   const size_t smem_k = tri(2 * P - 1) * sizeof(double2);
@@ -1733,8 +1751,9 @@ long long m2l_gemm64_system(Context &C, const FmmArgs &a, M2LGemmBufs &g, int4 s
     };
     products(0, ncls);
     auto reduce = [&](auto kernel) {
-      kernel<<<kNumSMs * 8, 256, 0, st>>>(a.m2l_off, cut[i].x, cut[i + 1].x, g.taken.p, g.Y64.p, qb, a.cell_x, t, P,
-                                          a.L64);
+      // Y64's first row is pair qb
+      kernel<<<kNumSMs * 8, 256, 0, st>>>(a.m2l_off, cut[i].x, cut[i + 1].x, g.taken.p,
+                                          g.Y64.p - (long long)qb * NDP, a.cell_x, t, P, a.L64);
       EXA_CHECK_LAUNCH();
     };
     if (NDP == 48) reduce(k_m2l_class_reduce<48, double>);
@@ -1750,7 +1769,7 @@ long long m2l_gemm64(Context &C, const FmmArgs &a, M2LGemmBufs &g, long long n_m
   const long long least = m2l_gemm64_pairs(a.P), nc = a.ncells;
   if (least <= 0 || n_m2l < least || nc <= 0) return n_m2l;
   cudaStream_t st = a.stream;
-  g.cnt.ensure(4);
+  g.cnt.ensure(5);
   std::vector<int4> systems;
   if (!a.nsys) {
     systems.push_back(make_int4(0, (int)nc, 0, (int)n_m2l));

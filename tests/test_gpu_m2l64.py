@@ -84,3 +84,19 @@ def test_the_workspace_changes_no_bit(ex, datasets, P, n, ncrit, dist):
     assert out[2][1] < out[1][1] < out[0][1]
     with ex.Fmm(**kw) as f, pytest.raises(ex.FmmError):
         f.set_m2l_workspace(0)
+
+
+@pytest.mark.parametrize("P", [8, 10])
+def test_few_pairs_a_class_go_pair_by_pair(ex, datasets, P):
+    """1.6M pairs in 51,000 offset classes: an operator for each would take 1.7 to 5 GB and longer
+    than the pairs themselves."""
+    x = datasets.plummer(150000, seed=5)
+    out = []
+    for _ in range(2):
+        with ex.Fmm(P=P, theta=0.3, ncrit=128, precision=ex.FP64) as f:
+            f.set_bodies(x)
+            f.solve()
+            assert f.info()["n_m2l"] >= 1500000
+            out.append(f.results())
+            assert f.device_bytes() < 1000e6
+    assert np.array_equal(*out)
