@@ -104,6 +104,8 @@ bool m2l_gemm(Context &C, const FmmArgs &a, M2LGemmBufs &g, long long n_m2l, int
 // number of pairs left, 0, all n_m2l (g's lists are then not set) or those in
 // left_off / left_src.
 long long m2l_gemm64(Context &C, const FmmArgs &a, M2LGemmBufs &g, long long n_m2l);
+// Device bytes of a solve of that many pairs through them, at most, with the default workspace.
+long long m2l_gemm64_bytes(int P, long long pairs);
 // The pairs outside the mixed policy compacted into g.comp_off / g.comp_src (CSR by target, list order).
 long long m2l_complement(Context &C, const FmmArgs &a, M2LGemmBufs &g, long long n_m2l, int min_level, int max_dl);
 

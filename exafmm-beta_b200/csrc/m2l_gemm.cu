@@ -1709,8 +1709,15 @@ long long m2l_gemm64_system(Context &C, const FmmArgs &a, M2LGemmBufs &g, int4 s
     else if (NDP == 64) launch(k_build_K<64, kKFp64>);
     else launch(k_build_K<112, kKFp64>);
   };
-  g.K64.ensure((long long)ncls * NDP * NDP);
-  build(0, ncls, nullptr);
+  // all of them once where they fit their share of the workspace; else a batch
+  // at a time, for each slab the ones it has pairs of
+  const long long op = (long long)NDP * NDP;
+  long long kcap = std::min<long long>(ncls, std::max<long long>(64, C.prm.m2l_work / 3 / (8 * op)));
+  while (!try_ensure(g.K64, kcap * op)) {
+    if (kcap <= 64) throw std::runtime_error("no device memory for the M2L operators");
+    kcap = std::max<long long>(kcap / 2, 64);
+  }
+  if (kcap >= ncls) build(0, ncls, nullptr);
   g.Ms64r.ensure(a.ncells * NDP);
   k_scale_M_real<<<kNumSMs * 8, 256, 0, st>>>(t, a.M64 + (long long)c0 * t.nterm, a.cell_x + c0, c1 - c0, P, nullptr,
                                               nullptr, g.Ms64r.p + (long long)c0 * NDP);
@@ -1749,7 +1756,15 @@ long long m2l_gemm64_system(Context &C, const FmmArgs &a, M2LGemmBufs &g, int4 s
       else if (NDP == 64) gemm64_launch<64>(g, k0, k1, sv, chunks_max, nd_of(P), st);
       else gemm64_launch<112>(g, k0, k1, sv, chunks_max, nd_of(P), st);
     };
-    products(0, ncls);
+    if (kcap >= ncls) {
+      products(0, ncls);
+    } else {
+      for (int k0 = 0; k0 < ncls; k0 += (int)kcap) {
+        const int k1 = (int)std::min<long long>(ncls, k0 + kcap);
+        build(k0, k1, g.cstart.p + k0);
+        products(k0, k1);
+      }
+    }
     auto reduce = [&](auto kernel) {
       // Y64's first row is pair qb
       kernel<<<kNumSMs * 8, 256, 0, st>>>(a.m2l_off, cut[i].x, cut[i + 1].x, g.taken.p,
@@ -1764,6 +1779,15 @@ long long m2l_gemm64_system(Context &C, const FmmArgs &a, M2LGemmBufs &g, int4 s
 }
 
 }  // namespace
+
+long long m2l_gemm64_bytes(int P, long long pairs) {
+  const long long least = m2l_gemm64_pairs(P), NDP = ndp_of(P);
+  if (least <= 0 || pairs < least) return 0;
+  const long long rows = std::min(pairs, kM2LWork * 2 / 3 / (8 * NDP));
+  // a slab's contributions and sort; the operators; per pair the class table (at
+  // most 12), its slot, the taken flag and the list of pairs left
+  return rows * (8 * NDP + 24) + std::min(pairs / 16 * NDP * NDP * 8, kM2LWork / 3) + 21 * pairs;
+}
 
 long long m2l_gemm64(Context &C, const FmmArgs &a, M2LGemmBufs &g, long long n_m2l) {
   const long long least = m2l_gemm64_pairs(a.P), nc = a.ncells;

@@ -29,6 +29,7 @@
 #include <cuda_runtime.h>
 
 #include "../../include/exafmm_b200.h"
+#include "fmm.h"
 
 namespace {
 
@@ -323,6 +324,7 @@ struct Request {
   unsigned long long seed = 0;
   const double *d_xyzq = nullptr; // a chain step's new positions in device memory (or null)
   long long est_bytes = 0;   // estimate at submission, then the bytes charged while in flight
+  long long est_work = 0;    // estimate of the work areas that a group shares
   Clock::time_point t_submit, t_start, t_end;
   double device_ms = 0;
   bool done = false;
@@ -362,14 +364,24 @@ struct exafmm_server {
   bool stop = false;
   std::vector<std::thread> threads;
 
-  // Upper estimate of a solve's device bytes: per body the bodies, keys,
-  // permutation, results and two-float copies, the cells' expansions and the
-  // interaction lists at their initial capacities; plus a fixed part.  A
-  // worker's context keeps its buffers, so a request is charged the larger of
-  // this and what that context already holds.
+  // Upper estimate of a solve's device bytes (theta >= 0.35, ncrit >= 64: longer
+  // lists outgrow their share of it; the mixed form's class products are not in
+  // it): per body the bodies, keys, permutation, results and two-float copies,
+  // the cells' expansions and the interaction lists, regrown once, and the P2P's
+  // segment sums; plus a fixed part.  The
+  // plain method's class products come on top, once for a context whatever its
+  // solve groups (est_work).  A worker's context keeps its buffers, so a request
+  // is charged the larger of this and what that context already holds.
   static long long estimate(long long n, int P) {
     const long long nt = (long long)P * (P + 1) / 2;
-    return n * (1400 + 24 * nt) + (64LL << 20);
+    return n * (1800 + 24 * nt) + std::min(8 * n + 65536, 1LL << 23) * 40 + (64LL << 20);
+  }
+  static long long estimate_work(long long n, const SolveParams &p) {
+    if (p.precision != EXAFMM_FP64) return 0;
+    // M2L pairs, a quarter above those of cubes and Plummer spheres at any
+    // theta and ncrit (about 4 n / ncrit cells with 11.5 / theta^3 each)
+    const double pairs = 58.0 * (double)n / ((double)p.ncrit * p.theta * p.theta * p.theta);
+    return exafmm_b200::m2l_gemm64_bytes(p.P, (long long)std::min(pairs, 2e9));
   }
 
   long long held_total(int except) const {
@@ -383,7 +395,7 @@ struct exafmm_server {
   // (which it then no longer holds idle), any other request the estimate or
   // the worker context it will use.
   long long charge_of(const Request *r, int w) const {
-    return r->sess ? std::max(r->est_bytes, r->sess->held) : std::max(r->est_bytes, held[w]);
+    return std::max(r->est_bytes + r->est_work, r->sess ? r->sess->held : held[w]);
   }
 
   // Head-of-line admission: the request fits beside what the other workers
@@ -438,16 +450,18 @@ struct exafmm_server {
           // the queued requests that can share this solve, in queue order,
           // each joining only if the group still fits the budget (the head
           // request alone is admitted as before)
-          long long bodies = r->n, est = r->est_bytes;
+          long long bodies = r->n, est = r->est_bytes, work = r->est_work;
           for (auto it = queue.begin(); it != queue.end() && (int)grp.size() < group_max;) {
             Request *q = *it;
             const long long est2 = est + q->est_bytes;
-            const long long charge2 = std::max(est2, held[w]);
+            const long long work2 = std::max(work, q->est_work);
+            const long long charge2 = std::max(est2 + work2, held[w]);
             if (!q->sess && q->n <= group_max_n && bodies + q->n <= group_bodies && same_params(q->prm, r->prm) &&
                 (double)(held_total(w) + in_flight + charge2) <= budget) {
               grp.push_back(q);
               bodies += q->n;
               est = est2;
+              work = work2;
               charge = charge2;
               it = queue.erase(it);
             } else {
@@ -902,6 +916,7 @@ int exafmm_server_submit(exafmm_server *s, const double *xyzq, long long n, doub
     if (s->stop) return 1;
     r->id = s->next_id++;
     r->est_bytes = s->estimate(n, P);
+    r->est_work = s->estimate_work(n, r->prm);
     *ticket = r->id;
     s->queue.push_back(r.get());
     s->reqs.emplace(r->id, std::move(r));
@@ -960,6 +975,7 @@ int exafmm_server_submit_step(exafmm_server *s, long long session, double sigma,
     r->t_submit = Clock::now();
     r->id = s->next_id++;
     r->est_bytes = s->estimate(q->n, q->prm.P);
+    r->est_work = s->estimate_work(q->n, q->prm);
     *ticket = r->id;
     s->queue.push_back(r.get());
     s->reqs.emplace(r->id, std::move(r));

@@ -100,6 +100,31 @@ def test_server_admission_serializes_under_tiny_budget(ex, datasets):
     s.close()
 
 
+@pytest.mark.parametrize("dist,n,P,theta", [("cube", 100000, 10, 0.4), ("plummer", 300007, 10, 0.35),
+                                            ("plummer", 400000, 8, 0.35)])
+def test_server_charges_what_a_plain_solve_holds(ex, datasets, dist, n, P, theta):
+    """Solves above the class products' line: their work areas are bounded and charged at admission."""
+    s = ex.Server(workers=1, hbm_budget_bytes=40e9)
+    s.wait(s.submit(getattr(datasets, dist)(n, seed=P), P=P, theta=theta, ncrit=64, precision=ex.FP64))
+    st = s.stats()
+    s.close()
+    assert 0 < st["held"] <= st["peak_admitted"]
+
+
+def test_a_group_is_charged_its_work_areas_once(ex, datasets):
+    x = datasets.cube(100000, seed=1)
+    kw = dict(P=10, theta=0.4, ncrit=64, precision=ex.FP64)
+    peak = []
+    for reps in (1, 6):
+        s = ex.Server(workers=1, hbm_budget_bytes=40e9)
+        s.set_grouping(64, 200000, 4 << 20)
+        for t in [s.submit(x, **kw) for _ in range(reps)]:
+            s.wait(t)
+        peak.append(s.stats()["peak_admitted"])
+        s.close()
+    assert peak[1] < 3 * peak[0]  # the first request may go alone, the others as a group
+
+
 def test_forest_batch_matches_single_solves(ex, datasets):
     """Forest mode: the systems of a call are grouped by size into forests, one
     context each; every system still gets the bits of its solo solve at its
