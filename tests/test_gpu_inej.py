@@ -69,6 +69,22 @@ def test_separate_sources_against_direct_and_reset(ex, datasets):
     g.close()
 
 
+@pytest.mark.parametrize("mixed", [False, True])
+def test_separate_sources_solve_again(ex, datasets, mixed):
+    x, jx = datasets.cube(3000, seed=4), datasets.cube(2500, seed=5)
+    with ex.Fmm(P=6, theta=0.4, ncrit=32, precision=ex.MIXED if mixed else ex.FP64) as f:
+        f.set_bodies(x)
+        f.set_sources(jx)
+        f.solve()
+        first = f.results()
+        f.solve()
+        assert np.array_equal(f.results(), first)
+        f.set_bodies(x)
+        f.solve()
+        assert np.array_equal(f.results(), first)
+        assert f.phase_times()["upward"] > 0
+
+
 def test_separate_sources_need_free_space(ex, datasets):
     x = datasets.cube(500, seed=1)
     f = ex.Fmm(P=6, images=1)
