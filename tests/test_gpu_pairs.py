@@ -103,3 +103,20 @@ def test_a_small_charge_very_near_does_not_overflow(ex, ns):
     for got in (ex.direct(t, s), solved):
         assert abs(got[0, 0] * d / q - 1.0) < 1e-10
         assert abs(got[0, 1] * d * d / q - 1.0) < 1e-10
+
+
+def test_reciprocal_distance_error(ex):
+    """1/r of one pair against the exact quotient, over r from 1e-150 to 1e150.  The distances have
+    26 bits, so that r^2 is exact.  Bound: the last addition rounds once, 2^-53, and e = 1 - r^2 y0^2
+    carries the rounding of r^2 y0, which counts half; the cubic term is below 2^-56 for the 20 bits
+    of y0 (a seed of 18 would do)."""
+    rng = np.random.default_rng(11)
+    n = 100000
+    m = rng.integers(1 << 25, 1 << 26, n)
+    d = np.ldexp(m.astype(np.float64), rng.integers(-500, 474, n))
+    t = np.zeros((n, 4))
+    t[:, 0] = d
+    got = ex.direct(t, np.array([[0.0, 0.0, 0.0, 1.0]]))[:, 0]
+    err = np.abs(got.astype(np.longdouble) * d.astype(np.longdouble) - 1)
+    print(f"largest error {float(err.max()):.3g}")
+    assert float(err.max()) < 1.5 * 2.0 ** -53 + 2.0 ** -56
