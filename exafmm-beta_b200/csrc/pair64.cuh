@@ -4,8 +4,9 @@
 
 namespace exafmm_b200 {
 
-// N pairs (separations d, charges q), pair i into the sums acc[i / PER]: the
-// potential, and the three that are subtracted from the gradient.
+// N pairs (separations d and charges q, which are used up), pair i into the sums
+// acc[i / PER]: the potential, and the three that are subtracted from the
+// gradient.
 //
 // 1 / sqrt(r2): the hardware's reciprocal square root of the high word (about
 // 20 bits) takes one third-order Householder step: with e = 1 - r2 y0^2,
@@ -17,11 +18,11 @@ namespace exafmm_b200 {
 //   * r2 = 0, every target's pair with itself: the charge is dropped, whatever
 //     it is (kernels/laplace.h:171 gives such a pair no weight, and an infinite
 //     or NaN charge times 0 would be NaN);
-//   * the others, which hardly ever come, take the library function and add
-//     their pair here as (q / r) / r / r: 1 / r^2 alone overflows for subnormal r2.
+//   * the others, which hardly ever come, take the library function and put the
+//     factors of 1/r into q and d: 1 / r^2 alone overflows for subnormal r2.
 template <int N, int PER>
-__device__ __forceinline__ void pairs64(const double (&dx)[N], const double (&dy)[N], const double (&dz)[N],
-                                        double (&q)[N], double (&acc)[N / PER][4]) {
+__device__ __forceinline__ void pairs64(double (&dx)[N], double (&dy)[N], double (&dz)[N], double (&q)[N],
+                                        double (&acc)[N / PER][4]) {
   double r2[N], inv[N];
   bool special = false;
 #pragma unroll
@@ -45,26 +46,20 @@ __device__ __forceinline__ void pairs64(const double (&dx)[N], const double (&dy
     if (rare) {
 #pragma unroll 1
       for (int i = 0; i < N; i++) {
-        double v = 1.0, x = 0.0, y = 0.0, z = 0.0, c = 0.0;
+        double v = r2[0];
 #pragma unroll
-        for (int k = 0; k < N; k++)
-          if (k == i && r2[k] != 0.0 && odd(r2[k])) {
-            v = r2[k];
-            x = dx[k];
-            y = dy[k];
-            z = dz[k];
-            c = q[k];
-            inv[k] = q[k] = 0.0;
-          }
-        const double r = rsqrt(v), s = c * r, s3 = s * r * r;
+        for (int k = 1; k < N; k++)
+          if (k == i) v = r2[k];
+        if (!odd(v) || v == 0.0) continue;
+        v = rsqrt(v);
 #pragma unroll
         for (int k = 0; k < N; k++)
           if (k == i) {
-            double(&a)[4] = acc[k / PER];
-            a[0] += s;
-            a[1] = fma(x, s3, a[1]);
-            a[2] = fma(y, s3, a[2]);
-            a[3] = fma(z, s3, a[3]);
+            q[k] *= v;
+            inv[k] = 1.0;
+            dx[k] = dx[k] * v * v;
+            dy[k] = dy[k] * v * v;
+            dz[k] = dz[k] * v * v;
           }
       }
     }
