@@ -212,23 +212,21 @@ __device__ __forceinline__ void p2p_finish(const P2PItems &w, P2PState &st, doub
   if (old != lf.y - 1) return;
   __threadfence();
   for (int i = threadIdx.x & 31; i < n; i += 32) {
-    double4 r = trg[first + i];
+    double t[4] = {0.0, 0.0, 0.0, 0.0};
     for (int s = 0; s < lf.z; s++) {
       const double *v = reinterpret_cast<const double *>(w.scratch + base + (long long)s * n + i);
-      r.x += __ldcg(v);
-      r.y -= __ldcg(v + 1);
-      r.z -= __ldcg(v + 2);
-      r.w -= __ldcg(v + 3);
+#pragma unroll
+      for (int k = 0; k < 4; k++) t[k] += __ldcg(v + k);
     }
-    trg[first + i] = r;
+    p2p_add(trg + first + i, t);
   }
 }
 
 // The sums of the pass's target j (lane-group member and slot) over one
 // segment: kept for p2p_finish, or added to the result at once (either way
-// segment by segment, in order).  Added up in shared memory instead, they took
-// 3 KB of a warp's 12 and the L1 that this leaves (mixed P2P of 4M bodies 17.54
-// against 17.38 ms).
+// segment by segment, in order: the results of a solve start from zero).  Added
+// up in shared memory instead, they took 3 KB of a warp's 12 and the L1 that
+// this leaves (mixed P2P of 4M bodies 17.54 against 17.38 ms).
 __device__ __forceinline__ void p2p_store(const P2PItems &w, P2PState &st, int j, const double (&v)[4],
                                           double4 *trg) {
   const int i = st.tb + j;
