@@ -59,7 +59,7 @@ struct P2PScan {
     const unsigned long long x = (unsigned long long)ns * (unsigned)slots;
     // segments: a rule on this leaf alone
     const unsigned long long c1 = (unsigned)seg_cost;
-    const unsigned long long sc = min(max(x / 2, c1), 8 * c1);
+    const unsigned long long sc = x > 32 * c1 ? 4 * c1 : min(max(x / 2, c1), 8 * c1);
     const int want = max(1, max((int)(sc / slots), ns / kMaxSeg));
     l.seg = (want + kSegAlign - 1) / kSegAlign * kSegAlign;
     l.nseg = (int)(((long long)ns + l.seg - 1) / l.seg);
@@ -122,11 +122,14 @@ P2PItems p2p_plan(Context &C, const FmmArgs &a, P2PWork &w, int tpl, int warps, 
   // a leaf of cost x is divided into at most x / (the item size) + 1 items
   v.cap = nc + (long long)warps * kSmallPerWarp + 1;
   v.ncells = nc;
-  // scratch of divided leaves: eight segments a body for the heavy ones, up to
-  // 2^23 slots (256 MB), and a quarter of that for the others
+  // scratch of divided leaves: every segment of every leaf for the heavy ones,
+  // up to 2^23 slots (256 MB).  In small trees of large leaves most are heavy:
+  // with eight segments a body many found no room and went whole (FP64 P2P of
+  // a 30,000-body Plummer sphere at ncrit 128 1.34 ms, 0.29 with it).  Two
+  // segments a body, up to 2^21 slots, for the others.
   P2PScan s;
-  s.scratch_heavy = std::min(std::min((long long)kMaxSeg * a.n, 8 * a.n + 65536), 1LL << 23);
-  s.scratch_small = s.scratch_heavy / 4;
+  s.scratch_heavy = std::min(kMaxSeg * a.n, 1LL << 23);
+  s.scratch_small = std::min(2 * a.n, 1LL << 21);
   w.items.ensure(kItemClasses * v.cap);
   w.leaf.ensure(nc);
   w.nsrc.ensure(nc);

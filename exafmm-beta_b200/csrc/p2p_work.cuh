@@ -7,13 +7,15 @@
 // (FP64) of a P2P phase whose arithmetic fills the GPU for 0.2 or 0.3 ms.  So
 //   * every leaf's source stream (the bodies of its list's leaves, one after
 //     another) is cut into segments by a fixed rule on the leaf alone: a
-//     multiple of kSegAlign sources, half the leaf within c to 8 c, in units c of
-//     the kernel's segment cost (target slots x sources), at most kMaxSeg
-//     segments; a leaf's result is the sum of its segments' sums in order.  The
-//     upper end, mixed P2P: 8 c against 4 c for leaves above 32 c takes 4M bodies
-//     from 17.38 to 17.34 ms and a 1M-charge water box from 4.47 to 4.40, at the
-//     same time on a 100,000-body cube, whose costly leaves need their segments
-//     shared out (a quarter of the leaf: 0.55 ms against 0.36; whole leaves 0.83);
+//     multiple of kSegAlign sources, in units c of the kernel's segment cost
+//     (target slots x sources) half the leaf within c to 8 c, 4 c for leaves
+//     above 32 c, at most kMaxSeg segments; a leaf's result is the sum of its
+//     segments' sums in order.  8 c above 32 c too would take the mixed P2P of 4M
+//     bodies from 17.38 to 17.34 ms and of a 1M-charge water box from 4.47 to
+//     4.41, but of 30,000 bodies on a sphere at ncrit 128 from 250 to 297 us and
+//     of a 90,000-charge box from 291 to 334: their costly leaves need their
+//     segments shared out (100,000-body cube: 0.36 ms; with quarters of such
+//     leaves 0.55, with whole leaves 0.83);
 //   * a leaf may be divided into items of whole segments, taken by different
 //     warps; these leave each segment's sums in scratch and the last warp to
 //     finish adds them in order.  A leaf taken whole adds its segments in the

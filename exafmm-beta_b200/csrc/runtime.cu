@@ -374,7 +374,7 @@ struct exafmm_server {
   // is charged the larger of this and what that context already holds.
   static long long estimate(long long n, int P) {
     const long long nt = (long long)P * (P + 1) / 2;
-    return n * (1800 + 24 * nt) + std::min(8 * n + 65536, 1LL << 23) * 40 + (64LL << 20);
+    return n * (1800 + 24 * nt) + std::min(66 * n, 10LL << 20) * 32 + (64LL << 20);
   }
   static long long estimate_work(long long n, const SolveParams &p) {
     if (p.precision != EXAFMM_FP64) return 0;
