@@ -9,8 +9,10 @@ namespace exafmm_b200 {
 enum Precision : int { kFP64 = 0, kMixed = 1 };
 
 // Default bytes of the plain method's class products: a slab's contributions
-// (two thirds) and a batch of operators (one third).
-constexpr long long kM2LWork = 3LL << 30;
+// and a batch of operators, half each.  The operators of 1M-body Plummer spheres
+// at P = 8 (27,000 to 37,000 classes) fit; a third of it, in batches built anew
+// for each slab, cost such a solve 0.5 of 13 ms of M2L.
+constexpr long long kM2LWork = 4LL << 30;
 
 struct Params {
   int P = 10;

@@ -282,22 +282,29 @@ __global__ void k_sys_ranges(const int *off, const int *sys_cell, int nsys, int 
   }
 }
 
-// Cuts targets [c0, c1) into slabs of at most `rows` pairs (or one target): out[i] = (first cell, first pair) of
-// slab i and, after the last, (c1, off[c1]).  One thread.
+// Cuts targets [c0, c1) into slabs of at most `rows` pairs (or one target): out[i]
+// = (first cell, first pair) of slab i and, after the last, (c1, off[c1]).  One warp.
 __global__ void k_slabs(const int *off, int c0, int c1, long long rows, int2 *out, int *n) {
+  const int lane = threadIdx.x;
   int k = 0;
   for (int c = c0; c < c1; k++) {
-    out[k] = make_int2(c, off[c]);
-    int lo = c + 1, hi = c1;  // last end with at most `rows` pairs
+    const int first = off[c];
+    if (lane == 0) out[k] = make_int2(c, first);
+    int lo = c + 1, hi = c1;  // the last end with at most `rows` pairs, 32 probes a step
     while (lo < hi) {
-      const int mid = lo + (hi - lo + 1) / 2;
-      if ((long long)off[mid] - off[c] <= rows) lo = mid;
-      else hi = mid - 1;
+      const int step = (hi - lo + 31) / 32;
+      const int at = (int)min((long long)lo + (long long)(lane + 1) * step, (long long)hi);
+      const int in = __popc(__ballot_sync(0xffffffffu, (long long)off[at] - first <= rows));
+      const int top = in == 32 ? hi : (int)min((long long)lo + (long long)(in + 1) * step, (long long)hi) - 1;
+      lo = (int)min((long long)lo + (long long)in * step, (long long)hi);
+      hi = top;
     }
     c = lo;
   }
-  out[k] = make_int2(c1, off[c1]);
-  *n = k;
+  if (lane == 0) {
+    out[k] = make_int2(c1, off[c1]);
+    *n = k;
+  }
 }
 
 // 3. Operator of each class: FP32 k-major, Kt[class][input dof][output dof]
@@ -1185,9 +1192,10 @@ k_m2l_class_mma_tma(const __grid_constant__ CUtensorMap msb_map, const int4 *chu
 // 128-byte runs.  Each output is
 // one FP64 sum over the inputs in order, whatever the chunk, so a pair's
 // contribution does not depend on the pairs beside it.  M2L phase, pair by pair
-// against products: 1M-body Plummer sphere at P = 8 (15.1M pairs) 31.4 -> 11.7
-// ms, of which these products 8.0 (42 % of the FP64 pipe); 100K-body cube at
-// P = 10 (0.6M pairs, about 90 a class) 3.27 -> 2.81 ms.
+// against products: 1M-body Plummer sphere at P = 8 (15.1M pairs, 550 a class)
+// 31.4 -> 11.7 ms; 100K-body cube at P = 10 (0.6M pairs, 90 a class) 3.25 -> 2.35.
+// FP64 pipe 46 % of active cycles at P = 8 (5.6M pairs of a 400K-body Plummer
+// sphere), 40 % on that cube, where the SMs are active 68 % of the launch.
 __host__ __device__ constexpr int gemm64_rows(int NDP) { return NDP > 64 ? 64 : 128; }
 __host__ __device__ constexpr int gemm64_bufs(int NDP) { return NDP > 64 ? 2 : 1; }
 __host__ __device__ constexpr size_t gemm64_smem_bytes(int NDP, int ND) {
@@ -1667,30 +1675,33 @@ long long m2l_gemm64_system(Context &C, const FmmArgs &a, M2LGemmBufs &g, int4 s
   k_pair_class64<<<kNumSMs * 8, 256, 0, st>>>(a.m2l_off, a.m2l_src, c0, c1, qb0, a.cell_x, a.cell_pl, g.hk.p, hcap - 1,
                                               limit, g.pair_slot.p, g.cnt.p);
   EXA_CHECK_LAUNCH();
+  // ---- slabs of whole targets, whose contributions fit the buffer
+  long long rows = std::min(np, std::max<long long>(np / kMaxSlabs + 1, C.prm.m2l_work / 2 / (8LL * NDP)));
   int *cnt = reinterpret_cast<int *>(C.pin + kPinScratch);
-  EXA_CUDA(cudaMemcpyAsync(cnt, g.cnt.p, 3 * sizeof(int), cudaMemcpyDeviceToHost, st));
-  EXA_CUDA(cudaStreamSynchronize(st));
+  std::vector<int2> cut{make_int2(c0, qb0), make_int2(c1, sys.w)};
+  auto read_counts = [&] {
+    int2 *slab = reinterpret_cast<int2 *>(C.pin + kPinScratch) + 2;
+    if (rows < np) {
+      g.slabs.ensure(2 * kMaxSlabs + 2);
+      k_slabs<<<1, 32, 0, st>>>(a.m2l_off, c0, c1, rows, g.slabs.p, g.cnt.p + 3);
+      EXA_CHECK_LAUNCH();
+      EXA_CUDA(cudaMemcpyAsync(slab, g.slabs.p, (2 * kMaxSlabs + 2) * sizeof(int2), cudaMemcpyDeviceToHost, st));
+    }
+    EXA_CUDA(cudaMemcpyAsync(cnt, g.cnt.p, 4 * sizeof(int), cudaMemcpyDeviceToHost, st));
+    EXA_CUDA(cudaStreamSynchronize(st));
+    if (rows < np) cut.assign(slab, slab + cnt[3] + 1);
+  };
+  read_counts();
   const int ncls = cnt[0];
   const long long taken = cnt[1];
   if (ncls <= 0 || ncls > limit || (long long)ncls * m2l_gemm64_places(P) > 32LL * cnt[2]) return 0;
-  // ---- slabs of whole targets, whose contributions fit the buffer; smaller
-  // ones where memory is short
-  long long rows = std::min(np, std::max<long long>(np / kMaxSlabs + 1, C.prm.m2l_work * 2 / 3 / (8LL * NDP)));
+  bool shorter = false;  // smaller slabs where memory is short
   while (!try_ensure(g.Y64, rows * NDP)) {
     if (rows <= np / kMaxSlabs + 1) throw std::runtime_error("no device memory for the M2L contributions");
     rows = std::max(rows / 2, np / kMaxSlabs + 1);
+    shorter = true;
   }
-  std::vector<int2> cut{make_int2(c0, qb0), make_int2(c1, sys.w)};
-  if (rows < np) {
-    g.slabs.ensure(2 * kMaxSlabs + 2);
-    k_slabs<<<1, 1, 0, st>>>(a.m2l_off, c0, c1, rows, g.slabs.p, g.cnt.p + 3);
-    EXA_CHECK_LAUNCH();
-    int2 *slab = reinterpret_cast<int2 *>(C.pin + kPinScratch) + 1;
-    EXA_CUDA(cudaMemcpyAsync(slab, g.slabs.p, (2 * kMaxSlabs + 2) * sizeof(int2), cudaMemcpyDeviceToHost, st));
-    EXA_CUDA(cudaMemcpyAsync(cnt, g.cnt.p + 3, sizeof(int), cudaMemcpyDeviceToHost, st));
-    EXA_CUDA(cudaStreamSynchronize(st));
-    cut.assign(slab, slab + *cnt + 1);
-  }
+  if (shorter) read_counts();
   const int nslab = (int)cut.size() - 1;
   long long most = 0;
   for (int i = 0; i < nslab; i++) most = std::max<long long>(most, cut[i + 1].y - cut[i].y);
@@ -1712,7 +1723,7 @@ long long m2l_gemm64_system(Context &C, const FmmArgs &a, M2LGemmBufs &g, int4 s
   // all of them once where they fit their share of the workspace; else a batch
   // at a time, for each slab the ones it has pairs of
   const long long op = (long long)NDP * NDP;
-  long long kcap = std::min<long long>(ncls, std::max<long long>(64, C.prm.m2l_work / 3 / (8 * op)));
+  long long kcap = std::min<long long>(ncls, std::max<long long>(64, C.prm.m2l_work / 2 / (8 * op)));
   while (!try_ensure(g.K64, kcap * op)) {
     if (kcap <= 64) throw std::runtime_error("no device memory for the M2L operators");
     kcap = std::max<long long>(kcap / 2, 64);
@@ -1783,10 +1794,10 @@ long long m2l_gemm64_system(Context &C, const FmmArgs &a, M2LGemmBufs &g, int4 s
 long long m2l_gemm64_bytes(int P, long long pairs) {
   const long long least = m2l_gemm64_pairs(P), NDP = ndp_of(P);
   if (least <= 0 || pairs < least) return 0;
-  const long long rows = std::min(pairs, kM2LWork * 2 / 3 / (8 * NDP));
+  const long long rows = std::min(pairs, kM2LWork / 2 / (8 * NDP));
   // a slab's contributions and sort; the operators; per pair the class table (at
   // most 12), its slot, the taken flag and the list of pairs left
-  return rows * (8 * NDP + 24) + std::min(pairs / 16 * NDP * NDP * 8, kM2LWork / 3) + 21 * pairs;
+  return rows * (8 * NDP + 24) + std::min(pairs / 16 * NDP * NDP * 8, kM2LWork / 2) + 21 * pairs;
 }
 
 long long m2l_gemm64(Context &C, const FmmArgs &a, M2LGemmBufs &g, long long n_m2l) {

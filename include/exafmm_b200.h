@@ -75,7 +75,7 @@ int exafmm_set_mixed_policy(exafmm_ctx *ctx, int m2l_fp32, int p2p_fp32, int min
  * (its P2P is a SIMD loop over targets, kernels/laplace.h:150-235). */
 int exafmm_set_p2p_targets_per_lane(exafmm_ctx *ctx, int tpl);
 /* Plain method: device bytes that the work areas of a large solve's M2L (its
- * per-class products) may take, at least 2^20; default 3 * 2^30.  A larger
+ * per-class products) may take, at least 2^20; default 4 * 2^30.  A larger
  * solve goes through them in pieces; the results do not depend on it. */
 int exafmm_set_m2l_workspace(exafmm_ctx *ctx, long long bytes);
 
@@ -280,7 +280,11 @@ int exafmm_kernel_p2p(long long ni, const double *xi, long long nj, const double
  * Both run a pool of `workers` solve contexts, each on its own host thread and
  * CUDA stream, so independent systems overlap on the GPU.  A system's results
  * do not depend on what else runs: every reduction of a solve has a fixed
- * order, so its bits are the same alone, in a batch or beside other requests. */
+ * order, so its bits are the same alone, in a batch or beside other requests.
+ * One exception, in the mixed form only: whether a forest's M2L takes the
+ * per-class products (exafmm_set_mixed_policy, m2l_fp32 1 and 4) goes by the
+ * pairs of the whole forest, so there a system of a large forest may differ
+ * from its solo solve within the precision bar. */
 typedef struct exafmm_batch exafmm_batch;
 int exafmm_batch_create(exafmm_batch **b, int P, double theta, int ncrit, int nspawn, int precision, int device,
                         int workers);
