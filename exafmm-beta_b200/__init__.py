@@ -246,7 +246,7 @@ class Fmm:
         self._check(lib().exafmm_set_p2p_targets_per_lane(self._h, int(tpl)))
 
     def set_m2l_workspace(self, nbytes: int):
-        """Device bytes of the plain method's M2L work areas (default 4 * 2^30); results do not depend on it."""
+        """Device bytes of the plain method's M2L work areas (default 6 * 2^30); results do not depend on it."""
         self._check(lib().exafmm_set_m2l_workspace(self._h, int(nbytes)))
 
     # ---- solve steps (examples/fmm.cxx:163-179) ----

@@ -9,10 +9,11 @@ namespace exafmm_b200 {
 enum Precision : int { kFP64 = 0, kMixed = 1 };
 
 // Default bytes of the plain method's class products: a slab's contributions
-// and a batch of operators, half each.  The operators of 1M-body Plummer spheres
-// at P = 8 (27,000 to 37,000 classes) fit; a third of it, in batches built anew
-// for each slab, cost such a solve 0.5 of 13 ms of M2L.
-constexpr long long kM2LWork = 4LL << 30;
+// and a batch of operators, half each.  1M-body Plummer spheres at P = 8 (15M
+// pairs, 27,000 to 37,000 classes, eight inputs): M2L 11.7 to 13.0 ms with 4 GB,
+// 11.5 to 12.8 with 6, 11.2 to 12.5 with 8 and 11.1 to 12.3 in one piece (11 GB);
+// 6 holds their operators, which built anew for each slab cost 0.5 ms.
+constexpr long long kM2LWork = 6LL << 30;
 
 struct Params {
   int P = 10;

@@ -75,7 +75,7 @@ int exafmm_set_mixed_policy(exafmm_ctx *ctx, int m2l_fp32, int p2p_fp32, int min
  * (its P2P is a SIMD loop over targets, kernels/laplace.h:150-235). */
 int exafmm_set_p2p_targets_per_lane(exafmm_ctx *ctx, int tpl);
 /* Plain method: device bytes that the work areas of a large solve's M2L (its
- * per-class products) may take, at least 2^20; default 4 * 2^30.  A larger
+ * per-class products) may take, at least 2^20; default 6 * 2^30.  A larger
  * solve goes through them in pieces; the results do not depend on it. */
 int exafmm_set_m2l_workspace(exafmm_ctx *ctx, long long bytes);
 
