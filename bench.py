@@ -270,7 +270,7 @@ def kernel_rooflines(P, mixed, n, info, phases, interactions, hbm_peak, peak_kin
                 "peak_kind": f"nominal CUDA-core FP32 (148 SMs x 128 lanes x 2 flop x {sm_mhz:.0f} MHz)",
                 "ms_per_launch": p2p_ms, "interactions": int(interactions),
                 "flops_per_interaction": P2P_FLOPS_PER_INTERACTION,
-                "note": "both P2P launches of a solve (FP32 in the mixed form, FP64 in the plain one)"})
+                "note": "the P2P launch of a solve (FP32 in the mixed form, FP64 in the plain one)"})
     m2l_ms = phases["m2l"]
     alg_flops = n_m2l * 8 * nt * P * P
     hbm("m2l", m2l_ms, n_m2l * (nt * cplx + 8) + C * 2 * nt * cplx,

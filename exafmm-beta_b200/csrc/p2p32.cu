@@ -8,22 +8,22 @@
 // A periodic image shift is added to the source's two-float pair when it is
 // staged (TwoSum of the hi parts, the rounding error carried into lo).
 //
-// Work mapping.  One warp evaluates one target leaf at a time.  The leaf's
-// source bodies (the bodies of every leaf in its P2P list, one after another)
-// form a stream that the warp stages into shared memory in chunks.  The 32
-// lanes are split into G = 32 / S groups of S lanes; each lane holds two
-// targets, so a group covers 2S targets, and the G groups take interleaved
-// pairs of the chunk's sources.  S is chosen from the leaf's size so that
-// small leaves still fill the warp (<= 8 bodies: 8 groups of 4 lanes; <= 16:
-// 4 x 8; <= 32: 2 x 16; larger: 1 x 32, in passes of 64 targets).  Two
-// consecutive sources go through one packed f32x2 operation, so the
-// arithmetic of two interactions is one instruction stream.
+// Work mapping.  One warp takes an item of one target leaf at a time: the whole
+// leaf, or some segments of its sources (p2p_work.cuh).  The leaf's source
+// bodies (the bodies of every leaf in its P2P list, one after another) form a
+// stream that the warp stages into shared memory in chunks.  The 32 lanes are
+// split into G = 32 / S groups of S lanes; each lane holds two or three targets,
+// so a group covers 2S or 3S of them, and the G groups take interleaved pairs of
+// the chunk's sources.  A pass takes the narrowest group that holds the targets
+// still left (at two a lane <= 8 bodies: 8 groups of 4 lanes; <= 16: 4 x 8;
+// <= 32: 2 x 16; larger: 1 x 32).  Two consecutive sources go through one packed
+// f32x2 operation, so the arithmetic of two interactions is one instruction stream.
 //
 // Accumulation.  Each lane sums a chunk (at most 32 sources per group) in
 // FP32 and then adds that partial into Kahan-compensated running sums
 // (include/kahan.h:34-48 semantics), so the error does not grow with the
-// number of chunks; the groups' sums are combined in FP64 and added to the
-// FP64 outputs.
+// number of chunks; at the end of a segment the groups' sums are combined in
+// FP64 and added to the FP64 outputs.
 //
 // r = 0.  A pair at zero distance contributes nothing, as in the reference
 // (kernels/laplace.h:171: invR2 = 0 when R2 = 0).  The test is applied to

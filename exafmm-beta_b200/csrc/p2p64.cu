@@ -10,7 +10,8 @@
 // memory in chunks of 32 G.  Every lane so holds targets in leaves of 8 to 64
 // bodies (the previous form, 32 lanes x 2 targets of one leaf, used 30-50 % of
 // its slots at the usual ncrit 64, called rsqrt(double) per pair, and one warp
-// served the longest list alone).
+// served the longest list alone).  1M-body Plummer sphere at ncrit 64 15.4 -> 4.57
+// ms, 100K-body cube 5.06 -> 0.46; the pipe 69 % busy.
 #include "p2p_work.cuh"
 #include "pair64.cuh"
 
