@@ -23,7 +23,7 @@ namespace {
 // added in order by k_direct_add, so the result does not depend on timing.
 // Bound: the FP64 pipe, 18 operations a pair (pair64.cuh).  4,096 targets x
 // 1,000,003 sources kept 16 of the 148 SMs busy with one thread per target and
-// every source (160 ms; 5.2 ms now, the pipe 75 % busy).
+// every source (160 ms; 5.2 ms now, the pipe 77 % busy).
 constexpr int kDirThreads = 128, kDirTile = 256;
 
 template <int TPL, bool IMAGES>

@@ -1194,7 +1194,7 @@ k_m2l_class_mma_tma(const __grid_constant__ CUtensorMap msb_map, const int4 *chu
 // contribution does not depend on the pairs beside it.  M2L phase, pair by pair
 // against products: 1M-body Plummer sphere at P = 8 (15.1M pairs, 550 a class)
 // 31.4 -> 11.7 ms; 100K-body cube at P = 10 (0.6M pairs, 90 a class) 3.25 -> 2.35.
-// FP64 pipe 46 % of active cycles at P = 8 (5.6M pairs of a 400K-body Plummer
+// FP64 pipe 47 % of active cycles at P = 8 (5.6M pairs of a 400K-body Plummer
 // sphere), 40 % on that cube, where the SMs are active 68 % of the launch.
 __host__ __device__ constexpr int gemm64_rows(int NDP) { return NDP > 64 ? 64 : 128; }
 __host__ __device__ constexpr int gemm64_bufs(int NDP) { return NDP > 64 ? 2 : 1; }
